@@ -33,10 +33,12 @@
 #include <algorithm>
 #include <climits>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace sseqs {
 namespace emb {
+
+using namespace tc;
 
 constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, GEMM_THREADS = 256;
 constexpr int LDK = BK + 8;        // [row][k] tile row, elements (80 B: ldmatrix conflict-free)
@@ -69,9 +71,6 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * 0.7978845608f * (1.f + 0.134145f * z * z);
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool pred) {
   const int n = pred ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
@@ -353,19 +352,6 @@ constexpr int TC_BM = 128, TC_BN = 256, TC_BK = 64, TC_STAGES = 2, TC_THREADS = 
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2, TC_B_BYTES = TC_BN * TC_BK * 2;
 constexpr int TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024;
-constexpr unsigned kWaitLimit = 1u << 26;
-
-// Shared-memory matrix descriptor: start, leading (K) and stride (MN)
-// byte offsets in 16-byte units, descriptor version 1, no swizzle.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;            // version
-  return d;                          // base offset 0, layout type 0 (no swizzle)
-}
-
 // Instruction descriptor, kind::f16: fp32 accumulate, bf16 A and B, both
 // K-major, M = 128, N = 256.
 constexpr uint32_t kIdescBf16 = (1u << 4)            // D format F32
@@ -373,19 +359,6 @@ constexpr uint32_t kIdescBf16 = (1u << 4)            // D format F32
                               | (1u << 10)           // B format BF16
                               | ((uint32_t)(TC_BN >> 3) << 17)
                               | ((uint32_t)(TC_BM >> 4) << 24);
-
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (unsigned i = 0; i < kWaitLimit; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
 
 template <int EPI>
 __global__ void __launch_bounds__(TC_THREADS, 2) gemm_tc_kernel(GemmArgs g, int* err) {
@@ -622,15 +595,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%2, %3}], [%4];"
       :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(mbar), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory");
 }
 
 // Fused epilogue of one row's 32 accumulator columns c0 .. c0 + 31.
@@ -1521,7 +1485,7 @@ using namespace sseqs::emb;
 static __device__ int g_tc_err;
 static bool g_tc_enabled = true;
 
-static int* tc_err_ptr() {
+int* sseqs::tc_error_flag() {
   static int* p[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -1536,7 +1500,7 @@ static int* tc_err_ptr() {
 template <int EPI>
 int launch_tc(const GemmArgs& g, cudaStream_t stream) {
   auto fn = gemm_tc_kernel<EPI>;
-  int* err = tc_err_ptr();
+  int* err = tc_error_flag();
   if (!err) return SSEQS_ERR_CUDA;
   if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)TC_SMEM) != cudaSuccess)
@@ -1603,7 +1567,7 @@ static bool ws_applies(const GemmArgs& g) {
 
 template <int EPI>
 int launch_tc_ws(const GemmArgs& g, cudaStream_t stream) {
-  int* err = tc_err_ptr();
+  int* err = tc_error_flag();
   if (!err) return SSEQS_ERR_CUDA;
   // A: lda-wide rows (the K tile at k0 is column k0 % lda of row m + k0 / lda)
   const int64_t a_len = g.lda >= g.K ? g.K : g.lda;
@@ -1629,10 +1593,10 @@ extern "C" int sseqs_gemm_set_tensor_path(int tcgen05) {
   return SSEQS_OK;
 }
 
-// Reads and clears the flag a tcgen05 GEMM sets when one of its bounded
-// waits runs out (synchronises the device).
+// Reads and clears the flag a tcgen05 kernel (GEMM, selection, prefilter)
+// sets when one of its bounded waits runs out (synchronises the device).
 extern "C" int sseqs_gemm_error(int* out) {
-  int* p = tc_err_ptr();
+  int* p = tc_error_flag();
   if (!p || !out) return SSEQS_ERR_ARG;
   int zero = 0;
   if (cudaMemcpy(out, p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return SSEQS_ERR_CUDA;
@@ -1848,7 +1812,7 @@ extern "C" int sseqs_score_select(const uint8_t* Q, int nq, const uint8_t* DB, i
   SelArgs a{Q, nq, DB, n, tau, count, cand, cand_score, cap};
   if (g_tc_enabled && n < (int64_t)INT32_MAX - 256) {
     // tcgen05: query tiles of N = the batch rounded up to 16 (at most 256)
-    int* err = tc_err_ptr();
+    int* err = tc_error_flag();
     if (!err) return SSEQS_ERR_CUDA;
     const int N = std::min(256, (nq + 15) / 16 * 16);
     const int qt = (nq + N - 1) / N;

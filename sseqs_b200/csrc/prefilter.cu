@@ -35,32 +35,17 @@
 // parked in a per-warp shared array until the segment's last row, when the
 // remaining diagonals (m >= Lt) are read off every column.
 //
-// Tensor-core form (rank k <= 4, N <= 2048; the reference's default rank is 4).
-// Only even lags enter the score, so with lags m = 32u + 2v (row u, column
-// v < 16) and target positions p = kk + 2v,
-//   c[32u + 2v] = sum_r sum_kk a_r[32u - kk] * b_r[kk + 2v],
-// a matrix product C[u, v] = sum_kk A[u, kk] B[kk, v] with
-//   A[u, kk] = a_r[32u - kk]   (the query factors read backwards: a row is 16
-//                                contiguous fp16 of the reversed query, rows
-//                                32 elements apart -- one shared copy per CTA,
-//                                loaded by ldmatrix at any (u, kk) offset),
-//   B[kk, v] = b_r[kk + 2v]    (the segment's factors: a fragment register is
-//                                one aligned half2 of the target array),
-// and the k ranks summed into the same accumulators.  mma.sync m16n8k16
-// (fp16 in, fp32 accumulate): a warp per segment, 16-row tiles of 512 lags,
-// K blocks of 16 target positions that meet the tile's non-zero band only,
-// two 8-column halves per A fragment.  The even-lag sums go to a per-warp
-// shared array, folded there (y[s] = c[s] + c[s+N]) into the maximum.  Work
-// is about (Lq + Lt) * Lt / 2 multiply-adds per rank against Lq * Lt / 2
-// useful ones; the factors are rounded to fp16 (the direct form rounds the
-// profile), sums stay fp32.
+// Tensor-core form (rank k <= 4; the reference's default rank is 4): the even
+// lags of the convolution as one matrix product per group of 128 segments on
+// tcgen05, D[segment, lag] = sum_(p, r) b_r[p] * a_r[(lag - p) mod N], see
+// prefilter_tc_kernel.
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <array>
 #include <utility>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace sseqs {
 namespace {
@@ -86,7 +71,6 @@ struct PfArgs {
   int k;
   int N;                    // cyclic length
   __half* out;              // [n]
-  int len_lo, len_hi;       // tensor-core form: segments with len_lo < min(len, N) <= len_hi
 };
 
 template <int C>
@@ -216,256 +200,570 @@ __global__ void __launch_bounds__(32 * PfShape<C>::WARPS) prefilter_kernel(PfArg
 }
 
 // ------------------------------------------------------- tensor-core form
-constexpr int kMmaRank = 4;            // ranks of the tensor-core form
-constexpr int kMmaPass = 4;            // 16-row tiles of 512 lags accumulated per pass
-constexpr int kQPad = 496;             // zero factors around the query (tile span - 16)
-constexpr int kTOff = 32;              // target factor of position p at [p + kTOff]
+// One matrix product per group of 128 segments: D[segment, lag] over the even
+// lags, K = (target position, rank), fp16 factors, fp32 accumulators in
+// tensor memory (128 lanes x up to 512 columns).
+//
+// Both operands use the no-swizzle K-major layout of 8-row x 16-byte core
+// matrices.  A 16-byte chunk of K holds 2 target positions x 4 ranks, so the
+// query operand needs no Toeplitz matrix: with arr[x] = (a_0 .. a_3)[-x mod N]
+// (8 bytes per x) row n of the operand is lag S - 2 - 2n and starts 16 bytes
+// after row n - 1, and the next chunk of K starts 16 bytes further too.  The
+// descriptors' strides (16 bytes from chunk to chunk, 128 from 8 rows to 8
+// rows) read the one 16N-byte array in place, for every lag and position; and
+// as arr is periodic in N, the cyclic fold y[s] = c[s] + c[s + N] happens in
+// the accumulation.
+//
+// A CTA (one per SM) takes every gridDim.x-th run of 32 segments, a window of
+// them at a time, and sorts the window by length (counting sort in shared
+// memory), so that the 128 segments of a group have nearly the same length:
+// a group costs its longest segment.  Warps 4-11 build the segment operand,
+// 32 positions to a 32 KB stage (one thread per segment: 32-byte loads, a
+// table of the 4 factors of every letter, replicated over the 32 lanes so that
+// no two lanes of a look-up share a bank); one thread of warp 12 issues the
+// MMAs; warps 0-3 read the accumulators (lane = segment, so the maximum over
+// lags needs no exchange between lanes).  Lags that a stage's positions
+// cannot reach are skipped in units of 16 columns, so the work follows
+// Lq * Lt, not the transform length.  A group of at most 256 even lags uses
+// half of the tensor memory, so that the next one's products overlap its
+// epilogue; one of more than 512 (N = 2048) takes two passes.
+//
+// Waits are bounded; one that runs out sets the error flag, the CTA stops
+// and its segments score NaN.
+//
+// Measured (300k segments of 30..1000 residues, rank 4) against the per-warp
+// mma.sync form it replaced, which built every segment's Toeplitz operand
+// (4600 warp instructions a segment): query length 858 2.04 -> 0.29 ms,
+// 100k segments at 1501 (N = 2048) 1.45 -> 0.23 ms.  At 858 the tensor pipe's
+// own time is 0.18 ms and shared memory, which feeds both operands and holds
+// the look-ups, is the next bound; below ~400 residues (0.15-0.17 ms) the issue of the
+// MMAs and the look-ups bound it.  tcgen05 runs the overlapping query
+// operand at its full rate (N = 256: 128 clocks per MMA, 64: 48).  A third
+// team of producers gained nothing.
+constexpr int kTcRank = 4;             // ranks of the tensor-core form
+constexpr int kTcGroup = 128;          // segments per group (MMA rows)
+constexpr int kTcPos = 32;             // target positions per stage
+constexpr int kTcStages = 4;
+constexpr int kTcStageBytes = kTcGroup * kTcPos * 8;
+constexpr int kTcWindow = 4096;        // segments sorted at a time
+constexpr int kTcCols = 512;           // tensor-memory columns (fp32 lags)
+constexpr int kTcEpiWarps = 4, kTcProducers = 2;      // producers: teams of 4 warps
+constexpr int kTcProdWarps = 4 * kTcProducers;
+constexpr int kTcThreads = 32 * (kTcEpiWarps + kTcProdWarps + 1);
+// look-up entries: bytes 64..95, then a position past the end, '-' or '*',
+// any other byte
+constexpr int kTcZero = 32, kTcGap = 33, kTcOther = 34, kTcEntries = 35;
+constexpr int kTcBins = 256;
+// Halves of the operands' shared-memory descriptors (fields as umma_desc):
+// the low one holds the start address and the K stride (segments: one chunk of
+// all 128; query: 16 bytes), the high one the 8-row stride (128 bytes) and the
+// version.
+constexpr uint32_t kDescLoA = (uint32_t)(kTcGroup * 16 / 16) << 16, kDescLoB = 1u << 16;
+constexpr uint32_t kDescHi = (128u >> 4) | (1u << 14);
 
-// Sizes for a longest cyclic length (and query, segment) MAXN.
-template <int MAXN, int W>
-struct PfMmaShape {
-  // reversed query factors per rank (fp16), whole 128-byte lines
-  static constexpr int QLEN = (MAXN + 2 * kQPad + 8 + 63) / 64 * 64;
-  // target factors per rank (fp16): positions -32 .. 128 * ceil((MAXN + 48) / 128) - 1,
-  // the span the fill writes (zero from len on) and the fragments read (< len + 46)
-  static constexpr int TLEN = kTOff + 128 * ((MAXN + 48 + 127) / 128);
-  // 16-row tiles of 512 lags covering Lq + len - 1 <= 2 MAXN - 1 lags
-  static constexpr int TILES = (2 * MAXN - 1 + 511) / 512;
-  static constexpr int LAGS = 256 * TILES;           // even lags per warp (fp32)
-  static constexpr size_t q_bytes = sizeof(__half) * kMmaRank * QLEN;
-  // the even-lag sums reuse the target factors' space once the products are done
-  static constexpr size_t warp_bytes = sizeof(__half) * kMmaRank * TLEN;
-  static_assert(warp_bytes >= sizeof(float) * LAGS && warp_bytes % 16 == 0, "warp space");
-  static constexpr size_t smem = q_bytes + W * warp_bytes + 256 + 16 * sizeof(__half) * 22;
+inline size_t tc_smem(int N) {
+  return (size_t)kTcStages * kTcStageBytes + (size_t)2 * N * 8 + kTcEntries * 32 * 8 +
+         kTcWindow * 2 + kTcBins * 4 + (kTcWindow / kTcGroup) * 4 + 128;
+}
+
+// Sizes of one group: even lags (rows of the query operand), stages, passes.
+struct TcGroup {
+  int S, R, stages, passes;
+  __device__ TcGroup(int N, int Lq, int longest) {
+    S = min(N, max(32, (Lq + longest - 1 + 31) & ~31));   // lags computed: 0 .. S - 1
+    R = S >> 1;
+    stages = max(1, (longest + kTcPos - 1) / kTcPos);
+    passes = (R + kTcCols - 1) / kTcCols;
+  }
 };
 
-// The rows of an A fragment are 64 bytes apart, so 16-byte chunk c of a
-// rank's query array is stored at chunk c ^ ((c >> 3) & 3) of its 128-byte
-// line: the 8 rows an ldmatrix reads then fall in 8 different bank groups.
-__device__ __forceinline__ int q_swz(int i) {
-  const int c = i >> 3;
-  return ((c ^ ((c >> 3) & 3)) << 3) | (i & 7);
-}
+__global__ void __launch_bounds__(kTcThreads, 1) prefilter_tc_kernel(PfArgs a, int* err) {
+  using namespace tc;
+  extern __shared__ __align__(128) unsigned char pf_sm[];
+  const int N = a.N, Lq = a.Lq, K = a.k;
+  unsigned char* stages = pf_sm;
+  uint2* arr = reinterpret_cast<uint2*>(stages + kTcStages * kTcStageBytes);   // [2N]
+  uint2* lut = arr + 2 * N;                                                    // [35][32]
+  uint16_t* order = reinterpret_cast<uint16_t*>(lut + kTcEntries * 32);
+  int* hist = reinterpret_cast<int*>(order + kTcWindow);
+  int* gmax = hist + kTcBins;
+  __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages];
+  __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], mma_done;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int valid_s;
+  __shared__ volatile int abort_s;
 
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
-                                          uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, "
-      "{%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-template <int MAXN, int W>
-__global__ void __launch_bounds__(32 * W) prefilter_mma_kernel(PfArgs a) {
-  using S = PfMmaShape<MAXN, W>;
-  constexpr int kQLen = S::QLEN, kTLen = S::TLEN;
-  extern __shared__ float4 smem_pf[];
-  __half* qf = reinterpret_cast<__half*>(smem_pf);                     // [4][kQLen]
-  uint8_t* wbase = reinterpret_cast<uint8_t*>(smem_pf) + S::q_bytes;
-  uint8_t* lut = wbase + W * S::warp_bytes;                           // [256]
-  __half* bx = reinterpret_cast<__half*>(lut + 256);                  // [4][22] (pad 16)
-  const int Lq = a.Lq, N = a.N, K = a.k;
-  // reversed query factors: ar_r[x] = a_r[-x] = A_r[qrev[-x]] for -(Lq-1) <= x <= 0,
-  // stored at [x + xoff]; xoff is a multiple of 8 so every ldmatrix row is aligned
-  const int xoff = (Lq - 1 + kQPad + 7) & ~7;
-  for (int i = threadIdx.x; i < kMmaRank * kQLen; i += blockDim.x) {
-    const int r = i / kQLen, li = i - r * kQLen, x = li - xoff;
-    float v = 0.f;
-    if (r < K && x <= 0 && x > -Lq) v = a.A[r * 21 + a.qrev[-x]];
-    qf[r * kQLen + q_swz(li)] = __float2half_rn(v);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int mma_warp = kTcEpiWarps + kTcProdWarps;
+  if (warp == mma_warp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&tmem_base_s)), "r"(kTcCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = (uint8_t)pf_pos((uint8_t)i);
-  for (int i = threadIdx.x; i < kMmaRank * 22; i += blockDim.x) {
-    const int r = i / 22, c = i - r * 22;
-    float v = 0.f;
-    if (r < K) v = c < 21 ? a.B[r * 21 + c] : (r + 1 < K ? a.B[(r + 1) * 21] : 0.f);
-    bx[i] = __float2half_rn(v);
+  if (tid == 0) {
+    auto init = [](uint64_t* b, int count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(b)), "r"(count));
+    };
+    for (int s = 0; s < kTcStages; ++s) { init(&full[s], 4); init(&empty[s], 1); }
+    for (int h = 0; h < 2; ++h) { init(&acc_full[h], 1); init(&acc_empty[h], kTcEpiWarps); }
+    init(&mma_done, 1);
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // query residues and factors, staged where the segment operand goes later
+  uint8_t* tq = stages;
+  __half* ta = reinterpret_cast<__half*>(stages + 2048);
+  for (int i = tid; i < Lq; i += kTcThreads) tq[i] = a.qrev[i];
+  for (int i = tid; i < kTcRank * 21; i += kTcThreads)
+    ta[i] = __float2half_rn(i / 21 < K ? a.A[i] : 0.f);
+  for (int i = tid; i < kTcEntries * 32; i += kTcThreads) {
+    const int e = i >> 5;
+    const int c = e == kTcGap ? 20 : e >= kTcZero ? 21 : pf_pos((uint8_t)(64 + e));
+    __half h[kTcRank];
+#pragma unroll
+    for (int r = 0; r < kTcRank; ++r) {
+      float v = 0.f;
+      if (r < K && e != kTcZero) v = c < 21 ? a.B[r * 21 + c] : (r + 1 < K ? a.B[(r + 1) * 21] : 0.f);
+      h[r] = __float2half_rn(v);
+    }
+    lut[i] = make_uint2(__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16),
+                        __half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16));
   }
   __syncthreads();
-
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  __half* tf = reinterpret_cast<__half*>(wbase + wib * S::warp_bytes);     // [4][kTLen]
-  float* lagbuf = reinterpret_cast<float*>(tf);                              // [S::LAGS]
-  const uintptr_t au = reinterpret_cast<uintptr_t>(a.ascii);
-  const uint32_t* abase = reinterpret_cast<const uint32_t*>(au & ~(uintptr_t)3);
-  const int64_t aoff = (int64_t)(au & 3);
-  const uint32_t qf_s = (uint32_t)__cvta_generic_to_shared(qf);
-  // ldmatrix x4: lane supplies row (lane & 7) + 8 * ((lane >> 3) & 1) of
-  // column block 8 * (lane >> 4)
-  const int lrow = (lane & 7) + 8 * ((lane >> 3) & 1), lcol = 8 * (lane >> 4);
-  const int g = lane >> 2, tq = lane & 3;
-  const int64_t nwarps = (int64_t)gridDim.x * W;
-
-  for (int64_t s = (int64_t)blockIdx.x * W + wib; s < a.n; s += nwarps) {
-    const int len = min((int)a.lengths[s], N);
-    if (len <= a.len_lo || len > a.len_hi) continue;     // another launch scores it
-    // positions -32 .. -1 are zero (the lag sums of the previous segment
-    // shared this space)
-    for (int i = lane; i < kMmaRank * (kTOff / 2); i += 32)
-      reinterpret_cast<__half2*>(tf + (i / (kTOff / 2)) * kTLen)[i % (kTOff / 2)] =
-          __float2half2_rn(0.f);
-    // target factors b_r[p] for p in [0, len + 48), zero from len on: lane l
-    // takes positions 4(l + 32m) .. +3, from the aligned words w and w + 1
-    // that hold them (w from this lane, w + 1 from the next one); all loads of
-    // the segment are issued before any is used, and a word is read only when
-    // it holds a byte of the segment
-    {
-      constexpr int kM = (MAXN + 48 + 127) / 128;
-      const int64_t ap = a.offsets[s] + aoff;
-      const int64_t w0 = ap >> 2;
-      const int64_t wend = (ap + len + 3) >> 2;          // words holding segment bytes
-      const uint32_t sh = (uint32_t)(ap & 3) * 8u;
-      const int nm = (len + 48 + 127) / 128;
-      uint32_t w[kM + 1];
-#pragma unroll
-      for (int m = 0; m <= kM; ++m) {
-        const int64_t wi = w0 + lane + 32 * m;
-        w[m] = (m <= nm && wi < wend) ? __ldg(abase + wi) : 0u;
-      }
-#pragma unroll
-      for (int m = 0; m < kM; ++m) {
-        if (m < nm) {
-          uint32_t nx = __shfl_down_sync(0xffffffffu, w[m], 1);
-          const uint32_t wrap = __shfl_sync(0xffffffffu, w[m + 1], 0);
-          if (lane == 31) nx = wrap;
-          const uint32_t raw = __funnelshift_r(w[m], nx, sh);
-          const int p0 = 4 * (lane + 32 * m);
-          int c[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) c[i] = p0 + i < len ? lut[(raw >> (8 * i)) & 0xffu] : -1;
-#pragma unroll
-          for (int r = 0; r < kMmaRank; ++r) {
-            __half h[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = c[i] >= 0 ? bx[r * 22 + c[i]] : __float2half_rn(0.f);
-            __half2* dst = reinterpret_cast<__half2*>(tf + r * kTLen + kTOff + p0);
-            dst[0] = __halves2half2(h[0], h[1]);
-            dst[1] = __halves2half2(h[2], h[3]);
-          }
-        }
-      }
+  for (int i = tid; i < 2 * N; i += kTcThreads) {
+    const int x = i - N, j = x <= 0 ? -x : N - x;       // a[-x mod N]
+    uint32_t v[2] = {0u, 0u};
+    if (j >= 0 && j < Lq) {
+      const int c = tq[j];
+      v[0] = __half_as_ushort(ta[c]) | ((uint32_t)__half_as_ushort(ta[21 + c]) << 16);
+      v[1] = __half_as_ushort(ta[42 + c]) | ((uint32_t)__half_as_ushort(ta[63 + c]) << 16);
     }
-    __syncwarp();
-    // lags 0 .. Lq + len - 2 in rows u = lag / 32, tiles of 16 rows, kMmaPass
-    // tiles per pass; each pass's sums stay in registers until the last pass
-    // is done, then go to lagbuf[16u + v] (even lag 32u + 2v), over the
-    // target factors
-    const int rows = (Lq + len - 1 + 31) / 32;
-    const int ntiles = (rows + 15) / 16;
-    float sums[S::TILES][2][4];
-#pragma unroll
-    for (int P = 0; P < S::TILES / kMmaPass; ++P) {
-      const int t0 = P * kMmaPass;
-      if (t0 < ntiles) {
-        // two accumulator sets (even and odd ranks) halve the chains of
-        // dependent MMAs
-        float acc[kMmaPass][2][2][4];
-#pragma unroll
-        for (int tj = 0; tj < kMmaPass; ++tj)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[tj][0][h][e] = acc[tj][1][h][e] = 0.f;
-        if (len > 0) {
-          // kk ranges over [-30, len); tile ti needs kk in (512 ti - Lq, 512 ti + 480]
-          const int kb_lo = max(-32, ((512 * t0 - Lq - 14) >> 4) << 4);
-          const int kb_hi = min(len - 1, 512 * (t0 + kMmaPass - 1) + 480);
-          for (int kb = kb_lo; kb <= kb_hi; kb += 16) {
-            uint32_t bf[kMmaRank][2][2];
-#pragma unroll
-            for (int r = 0; r < kMmaRank; ++r) {
-              const uint32_t* tr =
-                  reinterpret_cast<const uint32_t*>(tf + r * kTLen + kTOff + kb);
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int v = g + 8 * h;             // column: lag 32u + 2v
-                bf[r][h][0] = tr[tq + v];           // b[kb + 2tq + 2v .. +1]
-                bf[r][h][1] = tr[tq + v + 4];       // b[kb + 8 + 2tq + 2v .. +1]
-              }
-            }
-#pragma unroll
-            for (int tj = 0; tj < kMmaPass; ++tj) {
-              const int ti = t0 + tj;
-              if (ti < ntiles && kb + 15 > 512 * ti - Lq && kb <= 512 * ti + 480) {
-                // row u = 16 ti + lrow, columns kb + lcol .. +7: ar[kb + lcol - 32u ...]
-                const uint32_t qa =
-                    qf_s + 2u * (uint32_t)q_swz(kb + lcol - 32 * (16 * ti + lrow) + xoff);
-                uint32_t af[kMmaRank][4];
-#pragma unroll
-                for (int r = 0; r < kMmaRank; ++r)
-                  if (r < K) ldsm_x4(qa + (uint32_t)(2 * r * kQLen), af[r]);
-#pragma unroll
-                for (int r = 0; r < kMmaRank; ++r) {
-                  if (r < K) {
-                    mma_16816(acc[tj][r & 1][0], af[r], bf[r][0][0], bf[r][0][1]);
-                    mma_16816(acc[tj][r & 1][1], af[r], bf[r][1][0], bf[r][1][1]);
-                  }
-                }
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int tj = 0; tj < kMmaPass; ++tj)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sums[t0 + tj][h][e] = acc[tj][0][h][e] + acc[tj][1][h][e];
-      }
-    }
-    __syncwarp();                                // every lane's factor reads are done
-#pragma unroll
-    for (int ti = 0; ti < S::TILES; ++ti) {
-      if (ti < ntiles) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int u = 16 * ti + g + 8 * (e >> 1);
-            const int v = 2 * tq + (e & 1) + 8 * h;
-            lagbuf[16 * u + v] = sums[ti][h][e];
-          }
-        }
-      }
-    }
-    __syncwarp();
-    // y[s] = c[s] + c[s + N] over even s < N; lags past the computed tiles
-    // are 0, and so are lags no diagonal reaches
-    const int lim = 256 * ntiles;
-    float best = -INFINITY;
-    for (int e1 = lane; e1 < N / 2; e1 += 32) {
-      const int e2 = e1 + N / 2;
-      const float y = (e1 < lim ? lagbuf[e1] : 0.f) + (e2 < lim ? lagbuf[e2] : 0.f);
-      best = fmaxf(best, y);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (lane == 0) a.out[s] = __float2half_rn(0.5f * best);
-    __syncwarp();
+    arr[i] = make_uint2(v[0], v[1]);
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  auto fail = [&]() {
+    abort_s = 1;
+    atomicExch(err, 1);
+  };
+
+  // segment j of this CTA: runs of 32, gridDim.x apart
+  const int64_t runs = (a.n + 31) >> 5;
+  const int64_t mine = ((runs - blockIdx.x + gridDim.x - 1) / gridDim.x) << 5;
+  auto segment = [&](int64_t j) -> int64_t {
+    return ((((j >> 5) * gridDim.x) + blockIdx.x) << 5) + (j & 31);
+  };
+
+  // pipeline positions, kept by every role over all groups
+  uint32_t it = 0;                  // stages so far
+  uint32_t half = 0, uses[2] = {0, 0};
+  bool issued = false;
+  for (int64_t w0 = 0; w0 < mine; w0 += kTcWindow) {
+    // -------------------------------------------------- sort the window
+    const int cnt = (int)min((int64_t)kTcWindow, mine - w0);
+    for (int i = tid; i < kTcBins; i += kTcThreads) hist[i] = 0;
+    if (tid < kTcWindow / kTcGroup) gmax[tid] = 0;
+    __syncthreads();
+    auto length_of = [&](int64_t g) { return max(0, min((int)a.lengths[g], N)); };
+    auto bin_of = [](int len) { return kTcBins - 1 - min(kTcBins - 1, len >> 3); };
+    for (int i = tid; i < cnt; i += kTcThreads) {
+      const int64_t g = segment(w0 + i);
+      if (g < a.n) atomicAdd(&hist[bin_of(length_of(g))], 1);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int v[kTcBins / 32], sum = 0;
+#pragma unroll
+      for (int k = 0; k < kTcBins / 32; ++k) {
+        v[k] = hist[lane * (kTcBins / 32) + k];
+        sum += v[k];
+      }
+      int x = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) valid_s = x;
+      int run = x - sum;
+#pragma unroll
+      for (int k = 0; k < kTcBins / 32; ++k) {
+        hist[lane * (kTcBins / 32) + k] = run;
+        run += v[k];
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < cnt; i += kTcThreads) {
+      const int64_t g = segment(w0 + i);
+      if (g < a.n) {
+        const int len = length_of(g);
+        const int at = atomicAdd(&hist[bin_of(len)], 1);
+        order[at] = (uint16_t)i;
+        atomicMax(&gmax[at / kTcGroup], len);
+      }
+    }
+    __syncthreads();
+    const int valid = valid_s, groups = (valid + kTcGroup - 1) / kTcGroup;
+
+    if (warp >= kTcEpiWarps && warp < mma_warp) {
+      // ------------------------------------------------ segment operand
+      const uint32_t wg = (uint32_t)(warp - kTcEpiWarps) >> 2;   // team: every second stage
+      const int slot = (warp & 3) * 32 + lane;
+      // this thread's segment of a group (length 0 past the last one)
+      struct Seg { const uint8_t* src; int len; };
+      auto seg_of = [&](int g) -> Seg {
+        const int at = g * kTcGroup + slot;
+        if (g >= groups || at >= valid) return {a.ascii, 0};
+        const int64_t sg = segment(w0 + order[at]);
+        return {a.ascii + a.offsets[sg], length_of(sg)};
+      };
+      auto stages_of = [&](int g) {
+        const TcGroup G(N, Lq, gmax[g]);
+        return G.stages * G.passes;
+      };
+      // the bytes of a stage: the two aligned 32-byte chunks that cover its 32
+      // positions, read only where they hold a byte of the segment
+      struct Raw { uint32_t w[16]; };
+      auto fetch = [&](const Seg& s, int p0) -> Raw {
+        Raw r;
+        const uintptr_t at = (reinterpret_cast<uintptr_t>(s.src) & ~(uintptr_t)31) + p0;
+        const int sh = (int)(reinterpret_cast<uintptr_t>(s.src) & 31);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint32_t* w = r.w + 8 * k;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) w[q] = 0;
+          if (p0 < s.len && p0 + 32 * k - sh < s.len)
+            asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]),
+                           "=r"(w[6]), "=r"(w[7])
+                         : "l"(at + 32 * k));
+        }
+        return r;
+      };
+      // the bytes of the next stage and the next group's segment are fetched
+      // before the current stage is waited for, so that their latency is hidden
+      bool ok = true;
+      int g = 0, total = 0, t = 0;
+      Seg cur = {a.ascii, 0}, nxt = seg_of(0);
+      // (g, t) := the first stage at or after (g, t) in the order of stages
+      auto settle = [&]() {
+        while (g < groups && t >= total) {
+          t -= total;
+          ++g;
+          cur = nxt;
+          if (g < groups) total = stages_of(g);
+          nxt = seg_of(g + 1);
+        }
+      };
+      if (groups > 0) {
+        total = stages_of(0);
+        cur = nxt;
+        nxt = seg_of(1);
+        const uint32_t first = it;
+        t = (int)((wg + kTcProducers - first % kTcProducers) % kTcProducers);
+        uint32_t done = first + (uint32_t)t;   // stages done of this team's
+        settle();
+        Raw raw = {};
+        int p0 = 0;
+        if (g < groups) {
+          p0 = (t % max(1, TcGroup(N, Lq, gmax[g]).stages)) * kTcPos;
+          raw = fetch(cur, p0);
+        }
+        while (g < groups && ok) {
+          const Seg now = cur;
+          const int pos = p0;
+          uint32_t w[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) w[k] = raw.w[k];
+          t += kTcProducers;
+          settle();
+          if (g < groups) {
+            p0 = (t % TcGroup(N, Lq, gmax[g]).stages) * kTcPos;
+            raw = fetch(cur, p0);
+          }
+          const uint32_t stage = done % kTcStages;
+          if (!mbar_wait(smem_u32(&empty[stage]), ((done / kTcStages) & 1u) ^ 1u)) {
+            fail();
+            ok = false;
+          }
+          uint4* dst = reinterpret_cast<uint4*>(stages + stage * kTcStageBytes) + slot;
+          const int left = now.len - pos;       // positions of the segment from here on
+          if (left <= 0) {
+#pragma unroll
+            for (int c = 0; c < kTcPos / 2; ++c) dst[c * kTcGroup] = make_uint4(0, 0, 0, 0);
+          } else {
+            const int sh = (int)(reinterpret_cast<uintptr_t>(now.src) & 31);
+            if (sh & 16) {
+#pragma unroll
+              for (int k = 0; k < 12; ++k) w[k] = w[k + 4];
+            }
+            if (sh & 8) {
+#pragma unroll
+              for (int k = 0; k < 10; ++k) w[k] = w[k + 2];
+            }
+            if (sh & 4) {
+#pragma unroll
+              for (int k = 0; k < 9; ++k) w[k] = w[k + 1];
+            }
+            const uint32_t bits = (uint32_t)(sh & 3) * 8u;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = __funnelshift_r(w[k], w[k + 1], bits);
+            // bytes of word k before the end of the segment
+            auto keep = [&](int k) {
+              const int r = left - 4 * k;
+              return r >= 4 ? 0xffffffffu : r <= 0 ? 0u : (1u << (8 * r)) - 1u;
+            };
+            if (left < kTcPos) {
+#pragma unroll
+              for (int k = 0; k < 8; ++k) w[k] = (w[k] & keep(k)) | (0x40404040u & ~keep(k));
+            }
+            uint32_t odd = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) odd |= (w[k] ^ 0x40404040u) & 0xe0e0e0e0u;
+            if (odd == 0) {
+#pragma unroll
+              for (int k = 0; k < 8; ++k) w[k] &= 0x1f1f1f1fu;
+            } else {
+              // some byte is outside 64..95
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                uint32_t e = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                  const uint32_t c = (w[k] >> (8 * b)) & 0xffu;
+                  const uint32_t v = (c & 0xe0u) == 0x40u   ? (c & 31u)
+                                     : (c == '-' || c == '*') ? (uint32_t)kTcGap
+                                                              : (uint32_t)kTcOther;
+                  e |= v << (8 * b);
+                }
+                w[k] = e;
+              }
+            }
+            if (left < kTcPos) {                // past the end: the zero entry
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                w[k] = (w[k] & keep(k)) | ((uint32_t)kTcZero * 0x01010101u & ~keep(k));
+            }
+            const uint2* my = lut + lane;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const uint2 f0 = my[(w[k] & 0x3fu) * 32], f1 = my[((w[k] >> 8) & 0x3fu) * 32];
+              const uint2 f2 = my[((w[k] >> 16) & 0x3fu) * 32], f3 = my[(w[k] >> 24) * 32];
+              dst[(2 * k) * kTcGroup] = make_uint4(f0.x, f0.y, f1.x, f1.y);
+              dst[(2 * k + 1) * kTcGroup] = make_uint4(f2.x, f2.y, f3.x, f3.y);
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&full[stage]));
+          done += kTcProducers;
+          if (abort_s) ok = false;
+        }
+        // stages of the whole window, for the next one
+        for (int q = 0; q < groups; ++q) it += (uint32_t)stages_of(q);
+      }
+    } else if (warp == mma_warp) {
+      // ---------------------------------------------------- MMA issue
+      // The whole warp runs this loop and one elected lane's instructions
+      // take effect: with the values the same in every lane (broadcast
+      // explicitly where they come from memory) the compiler keeps the
+      // operands in uniform registers, where the instruction wants them.
+      bool ok = true;
+      const uint32_t leader = elect_one();
+      const uint32_t arr0 = smem_u32(arr) >> 4, stage0 = smem_u32(stages) >> 4;
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      for (int g = 0; g < groups && ok; ++g) {
+        const int longest = __shfl_sync(0xffffffffu, gmax[g], 0);
+        const TcGroup G(N, Lq, longest);
+        for (int p = 0; p < G.passes && ok; ++p) {
+          const int row0 = p * kTcCols, rows = min(kTcCols, G.R - row0);
+          const bool narrow = rows <= kTcCols / 2;
+          if (narrow ? !mbar_wait(smem_u32(&acc_empty[half]), (uses[half] & 1u) ^ 1u)
+                     : !(mbar_wait(smem_u32(&acc_empty[0]), (uses[0] & 1u) ^ 1u) &&
+                         mbar_wait(smem_u32(&acc_empty[1]), (uses[1] & 1u) ^ 1u))) {
+            fail();
+            ok = false;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t dcol = tm + (narrow ? half * (kTcCols / 2) : 0u) - (uint32_t)row0;
+          for (int t = 0; t < G.stages && ok; ++t, ++it) {
+            const uint32_t stage = it % kTcStages;
+            if (!mbar_wait(smem_u32(&full[stage]), (it / kTcStages) & 1u)) {
+              fail();
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t da = (stage0 + stage * (kTcStageBytes / 16)) | kDescLoA;
+            const int k0 = t * kTcPos;
+            const int nks = max(1, min(kTcPos / 4, (longest - k0 + 3) / 4));
+            // row r of the query operand at positions k0 ..: arr0 + (.. + 2r) / 2
+            const uint32_t db0 = (arr0 + (uint32_t)((N + k0 - (G.S - 2)) >> 1)) | kDescLoB;
+            // one MMA: rows from r0 of the query operand, K step ks (4
+            // positions: two chunks of the segment operand, 32 bytes of arr)
+            auto mma = [&](int r0, int ks, uint32_t idesc, uint32_t accum) {
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+                  "setp.ne.b32 p, %4, 0;\n\t"
+                  "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+                  "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}\n"
+                  :: "r"(dcol + (uint32_t)r0), "r"(da + (uint32_t)(ks * (2 * kTcGroup))),
+                     "r"(db0 + (uint32_t)(r0 + ks * 2)), "r"(idesc), "r"(accum), "n"(kDescHi));
+            };
+            // rows [r0, r1) times K steps [ka, kb); whole stages unrolled, as
+            // the issuing thread's own instructions are what bounds short
+            // queries
+            auto product = [&](int r0, int r1, int ka, int kb, uint32_t accum) {
+              r0 = max(r0, row0);
+              r1 = min(r1, row0 + rows);
+              for (; r0 < r1; r0 += 256) {
+                const uint32_t nn = (uint32_t)min(256, r1 - r0);
+                const uint32_t idesc = (1u << 4) | ((nn >> 3) << 17) |
+                                       ((uint32_t)(kTcGroup >> 4) << 24);
+                if (ka == 0 && kb == kTcPos / 4) {
+                  if (leader) {
+#pragma unroll
+                    for (int ks = 0; ks < kTcPos / 4; ++ks) mma(r0, ks, idesc, 1u);
+                  }
+                } else {
+                  for (int ks = ka; ks < kb; ++ks)
+                    if (leader) mma(r0, ks, idesc, accum);
+                }
+                __syncwarp();
+              }
+            };
+            int ka = 0;
+            if (t == 0) {            // the first step writes every column
+              product(0, G.R, 0, 1, 0u);
+              ka = 1;
+            }
+            // lags these positions reach: [k0, k0 + 31 + Lq - 1], and, past
+            // the end of the cycle, those up to k0 + 30 + Lq - N
+            const int hi = min(k0 + kTcPos - 2 + Lq, G.S - 2) & ~1;
+            const int rA0 = ((G.S - 2 - hi) >> 1) & ~15;
+            const int rA1 = min(G.R, (((G.S - 2 - k0) >> 1) + 16) & ~15);
+            product(rA0, rA1, ka, nks, 1u);
+            const int wrap = k0 + kTcPos - 2 + Lq - N;
+            if (wrap >= 0) {
+              const int rW0 = (max(0, G.S - 2 - (wrap & ~1)) >> 1) & ~15;
+              product(max(rW0, rA1), G.R, ka, nks, 1u);
+            }
+            commit_to(smem_u32(&empty[stage]), leader);
+            issued = true;
+          }
+          if (abort_s) ok = false;
+          if (narrow) {
+            commit_to(smem_u32(&acc_full[half]), leader);
+            ++uses[half];
+            half ^= 1u;
+          } else {
+            commit_to(smem_u32(&acc_full[0]), leader);
+            commit_to(smem_u32(&acc_full[1]), leader);
+            ++uses[0];
+            ++uses[1];
+          }
+        }
+      }
+      __syncwarp();
+    } else {
+      // ------------------------------------------------------ epilogue
+      const int slot = warp * 32 + lane;
+      bool ok = true;
+      for (int g = 0; g < groups && ok; ++g) {
+        const TcGroup G(N, Lq, gmax[g]);
+        float best = -INFINITY;
+        for (int p = 0; p < G.passes && ok; ++p) {
+          const int rows = min(kTcCols, G.R - p * kTcCols);
+          const bool narrow = rows <= kTcCols / 2;
+          const uint32_t h0 = narrow ? half : 0u, h1 = narrow ? half : 1u;
+          for (uint32_t h = h0; h <= h1; ++h) {
+            if (!mbar_wait(smem_u32(&acc_full[h]), uses[h] & 1u)) { fail(); ok = false; }
+            ++uses[h];
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) +
+                               (narrow ? half * (kTcCols / 2) : 0u);
+          for (int c = 0; c < rows; c += 32) {
+            uint32_t v[32];
+            // rows is a multiple of 16: the second half of the last read may
+            // lie past it, inside the allocation, and is not used
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,"
+                "%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, "
+                "[%32];"
+                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
+                  "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+                  "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]),
+                  "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                  "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
+                  "=r"(v[30]), "=r"(v[31])
+                : "r"(col + (uint32_t)c));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float m0 = __uint_as_float(v[0]), m1 = __uint_as_float(v[1]);
+#pragma unroll
+            for (int k = 2; k < 16; k += 2) {
+              m0 = fmaxf(m0, __uint_as_float(v[k]));
+              m1 = fmaxf(m1, __uint_as_float(v[k + 1]));
+            }
+            if (c + 16 < rows) {
+#pragma unroll
+              for (int k = 16; k < 32; k += 2) {
+                m0 = fmaxf(m0, __uint_as_float(v[k]));
+                m1 = fmaxf(m1, __uint_as_float(v[k + 1]));
+              }
+            }
+            best = fmaxf(best, fmaxf(m0, m1));
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            for (uint32_t h = h0; h <= h1; ++h) mbar_arrive(smem_u32(&acc_empty[h]));
+          if (narrow) half ^= 1u;
+        }
+        const int at = g * kTcGroup + slot;
+        if (at < valid) {
+          const int64_t sg = segment(w0 + order[at]);
+          // even lags that no diagonal reaches have y = 0
+          if (Lq + length_of(sg) - 1 <= N - 2) best = fmaxf(best, 0.f);
+          a.out[sg] = __float2half_rn(0.5f * best);
+        }
+        if (abort_s) ok = false;
+      }
+    }
+    __syncthreads();
+    if (abort_s) break;
+  }
+  // every MMA issued is complete before the tensor memory is freed
+  if (issued) {
+    commit_to(smem_u32(&mma_done), elect_one());
+    if (!mbar_wait(smem_u32(&mma_done), 0)) fail();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (abort_s) {
+    for (int64_t j = tid; j < mine; j += kTcThreads) {
+      const int64_t sg = segment(j);
+      if (sg < a.n) a.out[sg] = __ushort_as_half((unsigned short)0x7fff);
+    }
+  }
+  if (warp == mma_warp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTcCols));
 }
 
-template <int MAXN, int W>
-int launch_pf_mma(const PfArgs& a, cudaStream_t stream) {
-  using S = PfMmaShape<MAXN, W>;
-  static_assert(S::TILES % kMmaPass == 0, "whole passes");
-  const void* fn = (const void*)prefilter_mma_kernel<MAXN, W>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem) !=
-      cudaSuccess)
+int launch_pf_tc(const PfArgs& a, cudaStream_t stream) {
+  int* err = tc_error_flag();
+  if (!err) return SSEQS_ERR_CUDA;
+  const size_t smem = tc_smem(a.N);
+  if (cudaFuncSetAttribute((const void*)prefilter_tc_kernel,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return SSEQS_ERR_CUDA;
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * W, S::smem) != cudaSuccess ||
-      nb < 1)
-    return SSEQS_ERR_CUDA;
-  const int64_t need = (a.n + W - 1) / W;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)device_sm_count() * nb));
-  { prefilter_mma_kernel<MAXN, W><<<grid, 32 * W, S::smem, stream>>>(a); count_launches(1); }
+  const int64_t groups = (a.n + kTcGroup - 1) / kTcGroup;
+  const int grid = (int)std::min<int64_t>(groups, device_sm_count());
+  { prefilter_tc_kernel<<<grid, kTcThreads, smem, stream>>>(a, err); count_launches(1); }
   return status_of(cudaGetLastError());
 }
 
@@ -483,25 +781,10 @@ std::array<PfInfo, sizeof...(I)> pf_table(std::integer_sequence<int, I...>) {
 }
 
 int launch_pf(const PfArgs& a, cudaStream_t stream) {
-  // tensor-core form for ranks up to 4: segments and queries up to 1024
-  // residues with 16 warps per CTA; longer ones (cyclic length 2048) with the
-  // bigger buffers of the 2048 form, 8 warps per CTA
-  if (a.k <= kMmaRank && a.Lq >= 1 && a.N <= 2048) {
-    if (a.Lq <= 1024) {
-      PfArgs b = a;
-      b.len_lo = -1;
-      b.len_hi = 1024;
-      const int st = launch_pf_mma<1024, 16>(b, stream);
-      if (st != SSEQS_OK || a.N <= 1024) return st;
-      b.len_lo = 1024;
-      b.len_hi = a.N;
-      return launch_pf_mma<2048, 8>(b, stream);
-    }
-    PfArgs b = a;
-    b.len_lo = -1;
-    b.len_hi = a.N;
-    return launch_pf_mma<2048, 8>(b, stream);
-  }
+  // Ranks up to 4 fit the 16-byte operand chunks of the tensor-core form,
+  // which is faster at every size (its note has the figures); higher ranks and
+  // empty queries take the direct sums.
+  if (a.k <= kTcRank && a.Lq >= 1) return launch_pf_tc(a, stream);
   static const auto table = pf_table(std::make_integer_sequence<int, 64>{});
   const int C = std::max(1, (a.Lq + 31) / 32);
   const PfInfo& info = table[C - 1];
@@ -542,6 +825,6 @@ extern "C" int sseqs_prefilter(const uint8_t* ascii, const int64_t* offsets, con
   if (!workspace || ws_bytes < sseqs_prefilter_workspace_bytes(n, k)) return SSEQS_ERR_WORKSPACE;
   if (n_segments == 0) return SSEQS_OK;
   PfArgs a{ascii, offsets, lengths, n_segments, lut_a, lut_b, query_pos_reversed, query_len, k, n,
-           reinterpret_cast<__half*>(out_scores), -1, n};
+           reinterpret_cast<__half*>(out_scores)};
   return launch_pf(a, stream);
 }

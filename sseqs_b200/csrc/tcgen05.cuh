@@ -1,0 +1,74 @@
+// Building blocks of the tcgen05 kernels: mbarrier waits, shared-memory
+// matrix descriptors, and the flag their bounded waits set.
+#pragma once
+#include "common.cuh"
+
+namespace sseqs {
+
+// Device flag of the current device that a kernel sets when one of its
+// bounded waits runs out (read and cleared by sseqs_gemm_error); null on error.
+int* tc_error_flag();
+
+namespace tc {
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+constexpr unsigned kWaitLimit = 1u << 26;
+
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+  for (unsigned i = 0; i < kWaitLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(mbar), "r"(bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory");
+}
+
+// 1 in one lane of a converged warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(r));
+  return r;
+}
+
+// Arrival on `mbar` when the MMAs issued so far are done (from the lane whose
+// `leader` is set; the lane must have issued them).
+__device__ __forceinline__ void commit_to(uint32_t mbar, uint32_t leader) {
+  if (leader)
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                 :: "r"(mbar) : "memory");
+  __syncwarp();
+}
+
+// Shared-memory matrix descriptor: start, leading (K) and stride (MN)
+// byte offsets in 16-byte units, descriptor version 1, no swizzle.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
+  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
+  d |= (uint64_t)1 << 46;            // version
+  return d;                          // base offset 0, layout type 0 (no swizzle)
+}
+
+}  // namespace tc
+}  // namespace sseqs
