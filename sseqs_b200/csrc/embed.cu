@@ -860,6 +860,76 @@ __global__ void conv1_table_kernel(const uint8_t* cls, int64_t P, const float* T
   }
 }
 
+// The same for D = 256, a warp to 32 consecutive rows.  Lane l holds channels
+// 4l .. 4l + 3 and 128 + 4l .. + 3, so its two 16-byte table reads per tap are
+// conflict-free (8 adjacent channels per lane, as above, cost twice the
+// wavefronts) and the row's class is the same for the whole warp: classes are
+// read 32 at a time and broadcast, a padding tap costs no read, and bias and
+// addresses are formed once.  Sums in the same order as above.  Bound by
+// shared memory: 5 table rows of 1 KB for each 512-byte output row.
+// Measured on 5.9M rows: 4.63 -> 1.56 ms (shared-memory floor 0.84, about 150
+// instructions a row 0.8, output writes 0.46).
+constexpr int kConvWarps = 16;
+__global__ void __launch_bounds__(32 * kConvWarps, 2)
+    conv1_table256_kernel(const uint8_t* cls, int64_t P, const float* T, const float* bias,
+                          const uint8_t* mask, __nv_bfloat16* Y, __nv_bfloat16* Z) {
+  constexpr int D = 256;
+  extern __shared__ float4 t_sm[];
+  for (int i = threadIdx.x; i < 5 * 21 * D / 4; i += blockDim.x)
+    t_sm[i] = reinterpret_cast<const float4*>(T)[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const float4 b0 = reinterpret_cast<const float4*>(bias)[lane];
+  const float4 b1 = reinterpret_cast<const float4*>(bias)[lane + 32];
+  auto class_at = [&](int64_t q) { return q >= 0 && q < P ? (int)cls[q] : 255; };
+  const int64_t step = (int64_t)gridDim.x * kConvWarps * 32;
+  for (int64_t p0 = ((int64_t)blockIdx.x * kConvWarps + (threadIdx.x >> 5)) * 32; p0 < P;
+       p0 += step) {
+    // classes of rows p0 - 2 .. p0 + 33
+    const int ca = class_at(p0 - 2 + lane), cb = lane < 4 ? class_at(p0 + 30 + lane) : 255;
+    const bool keep_l = p0 + lane < P && (mask ? mask[p0 + lane] != 0 : true);
+    const unsigned keep_m = __ballot_sync(0xffffffffu, keep_l);
+    const int rows = (int)min((int64_t)32, P - p0);
+    auto cls_of = [&](int k) {           // class of row p0 - 2 + k, k warp-uniform
+      return k < 32 ? __shfl_sync(0xffffffffu, ca, k) : __shfl_sync(0xffffffffu, cb, k - 32);
+    };
+    int k[5];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) k[t + 1] = cls_of(t);
+    for (int r = 0; r < rows; ++r) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) k[t] = k[t + 1];
+      k[4] = cls_of(r + 4);
+      float4 z0 = b0, z1 = b1;
+#pragma unroll
+      for (int t = 0; t < 5; ++t) {
+        if (k[t] < 21) {
+          const float4* tr = t_sm + (t * 21 + k[t]) * (D / 4) + lane;
+          const float4 a = tr[0], b = tr[32];
+          z0.x += a.x; z0.y += a.y; z0.z += a.z; z0.w += a.w;
+          z1.x += b.x; z1.y += b.y; z1.z += b.z; z1.w += b.w;
+        }
+      }
+      const bool keep = (keep_m >> r) & 1u;
+      const float z[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
+      __align__(8) __nv_bfloat16 zy[8], yy[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        zy[j] = __float2bfloat16_rn(keep ? z[j] : 0.f);
+        yy[j] = __float2bfloat16_rn(keep ? gelu_f(__bfloat162float(zy[j])) : 0.f);
+      }
+      uint2* y = reinterpret_cast<uint2*>(Y + (p0 + r) * D) + lane;
+      y[0] = reinterpret_cast<const uint2*>(yy)[0];
+      y[32] = reinterpret_cast<const uint2*>(yy)[1];
+      if (Z) {
+        uint2* zp = reinterpret_cast<uint2*>(Z + (p0 + r) * D) + lane;
+        zp[0] = reinterpret_cast<const uint2*>(zy)[0];
+        zp[32] = reinterpret_cast<const uint2*>(zy)[1];
+      }
+    }
+  }
+}
+
 // X0[p][c] = E[cls[p]][c] for real rows (cls < 21), 0 for padding (cls 255).
 __global__ void embed_lookup_kernel(const uint8_t* cls, int64_t P, const __nv_bfloat16* E, int D,
                                     __nv_bfloat16* X) {
@@ -884,16 +954,54 @@ __global__ void embed_grad_kernel(const uint8_t* cls, int64_t P, const __nv_bflo
   }
 }
 
+// Sum over rows [0, n) of 8 channels a lane (lane l: 8l ..), rows warp, warp +
+// nwarps, .., added over the block's warps: part[warp][channel] in shared memory.
+// 16-byte loads, four in flight per lane.
+__device__ __forceinline__ void sum_rows256(const __nv_bfloat16* y, int n, int warp, int nwarps,
+                                            int lane, float (*part)[256]) {
+  float acc[8] = {};
+  const uint4* src = reinterpret_cast<const uint4*>(y) + lane;
+  auto add = [&](const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      acc[2 * h] += __uint_as_float(w[h] << 16);
+      acc[2 * h + 1] += __uint_as_float(w[h] & 0xffff0000u);
+    }
+  };
+  int p = warp;
+  for (; p + 3 * nwarps < n; p += 4 * nwarps) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = src[(int64_t)(p + i * nwarps) * 32];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) add(v[i]);
+  }
+  for (; p < n; p += nwarps) add(src[(int64_t)p * 32]);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) part[warp][8 * lane + j] = acc[j];
+}
+
 // One block of D = blockDim.x threads per sequence: pooled = mean of its
-// rows, emb = pooled / |pooled|.
+// rows, emb = pooled / |pooled|.  D = 256 (16-byte aligned Y) sums with 16-byte loads, 8 warps
+// on different rows (one 2-byte load per thread and row, as other widths do, left too
+// few bytes in flight: 5.9M rows 0.71 ms, now 0.47; reading them once takes 0.46).
 __global__ void pool_normalize_kernel(const __nv_bfloat16* Y, const int64_t* start,
                                       const int32_t* len, float* pooled, float* emb,
                                       float* inv_norm) {
   const int s = blockIdx.x, c = threadIdx.x, D = blockDim.x;
   const int n = len[s];
-  const __nv_bfloat16* y = Y + start[s] * D + c;
+  __shared__ float part[8][256];
   float acc = 0.f;
-  for (int p = 0; p < n; ++p) acc += __bfloat162float(y[(int64_t)p * D]);
+  if (D == 256 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0) {
+    sum_rows256(Y + start[s] * D, n, c >> 5, 8, c & 31, part);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) acc += part[w][c];
+  } else {
+    const __nv_bfloat16* y = Y + start[s] * D + c;
+    for (int p = 0; p < n; ++p) acc += __bfloat162float(y[(int64_t)p * D]);
+  }
   const float mean = n > 0 ? acc / (float)n : 0.f;
   __shared__ float red[32];
   float sq = mean * mean;
@@ -966,8 +1074,38 @@ __global__ void pool_backward_kernel(const float* emb, const float* dE, const fl
   __syncthreads();
   const int n = len[s];
   const float dp = (g - e * red[0]) * inv_norm[s] / (float)max(n, 1);
-  const int64_t base = start[s] * D + c;
   const __nv_bfloat16 gb = __float2bfloat16_rn(dp);
+  if (D == 256 && ((reinterpret_cast<uintptr_t>(Z) | reinterpret_cast<uintptr_t>(dZ) |
+                    reinterpret_cast<uintptr_t>(G)) & 15) == 0) {
+    // 8 channels a lane, a row a warp: 16-byte loads and stores (a training
+    // step's 0.4M rows: 534 -> 156 us)
+    __shared__ float dps[256];
+    __shared__ __align__(16) __nv_bfloat16 gbs[256];
+    dps[c] = dp;
+    gbs[c] = gb;
+    __syncthreads();
+    const int lane = c & 31;
+    float d8[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) d8[j] = dps[8 * lane + j];
+    const uint4 g8 = reinterpret_cast<const uint4*>(gbs)[lane];
+    for (int p = c >> 5; p < n; p += 8) {
+      const int64_t i = (start[s] + p) * 32 + lane;
+      const uint4 z = reinterpret_cast<const uint4*>(Z)[i];
+      const uint32_t w[4] = {z.x, z.y, z.z, z.w};
+      __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        o[2 * h] = __float2bfloat16_rn(d8[2 * h] * gelu_grad(__uint_as_float(w[h] << 16)));
+        o[2 * h + 1] =
+            __float2bfloat16_rn(d8[2 * h + 1] * gelu_grad(__uint_as_float(w[h] & 0xffff0000u)));
+      }
+      reinterpret_cast<uint4*>(dZ)[i] = *reinterpret_cast<const uint4*>(o);
+      if (G) reinterpret_cast<uint4*>(G)[i] = g8;
+    }
+    return;
+  }
+  const int64_t base = start[s] * D + c;
   for (int p = 0; p < n; ++p) {
     const int64_t i = base + (int64_t)p * D;
     dZ[i] = __float2bfloat16_rn(dp * gelu_grad(__bfloat162float(Z[i])));
@@ -1684,6 +1822,18 @@ extern "C" int sseqs_embed_conv1_table(const uint8_t* cls, int64_t P, const floa
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (!al(T) || !al(Y) || (Z && !al(Z))) return SSEQS_ERR_ARG;
   const size_t smem = sizeof(float) * 5 * 21 * (size_t)D;
+  if (D == 256 && al(bias)) {
+    if (cudaFuncSetAttribute((const void*)conv1_table256_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return SSEQS_ERR_CUDA;
+    const int blocks = (int)std::min<int64_t>((P + 32 * kConvWarps - 1) / (32 * kConvWarps),
+                                              (int64_t)device_sm_count() * 2);
+    { conv1_table256_kernel<<<blocks, 32 * kConvWarps, smem, stream>>>(
+          cls, P, T, bias, row_mask, static_cast<__nv_bfloat16*>(Y),
+          static_cast<__nv_bfloat16*>(Z));
+      count_launches(1); }
+    return status_of(cudaGetLastError());
+  }
   if (cudaFuncSetAttribute((const void*)conv1_table_kernel,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return SSEQS_ERR_CUDA;
