@@ -369,6 +369,19 @@ int sseqs_embed_lookup(const uint8_t* cls, int64_t P, const void* E, int D, void
 /* dE[cls[p]][c] += dX[p][c] (fp32 dE, bf16 dX). */
 int sseqs_embed_grad(const uint8_t* cls, int64_t P, const void* dX, int D, float* dE,
                      cudaStream_t stream);
+/* Gradients through the first convolution and the residue embedding: with
+ * G[t][k][co] = sum of dZ[p][co] over rows p with cls[p - 2 + t] == k (rows
+ * outside [0, P) and classes >= 21 contribute nothing),
+ *   dWT[(t * cin + ci)][co] += sum_k E[k][ci] G[t][k][co],
+ *   dE[k][ci] += sum_t sum_co Wf[ci][4 - t][co] G[t][k][co].
+ * cls uint8 [P]; dZ bf16 [P x D], D = 256; E bf16 [21 x cin]; Wf bf16
+ * [cin][5][D] (the layout sseqs_adam_conv writes); G: workspace of 5 * 21 * D
+ * floats, left holding the sums.  Stands for the weight- and data-gradient GEMMs of
+ * that layer and sseqs_embed_grad. */
+int sseqs_embed_conv1_grad(const uint8_t* cls, int64_t P, const void* dZ, int D, const void* E,
+                           int cin, const void* Wf, float* G, float* dWT, float* dE,
+                           cudaStream_t stream);
+
 /* Per sequence s: pooled = mean of rows start[s] .. + len[s] of Y [P x D]
  * (bf16), emb = pooled / |pooled|, inv_norm = 1 / |pooled| (fp32). */
 int sseqs_pool_normalize(const void* Y, int D, const int64_t* start, const int32_t* len,

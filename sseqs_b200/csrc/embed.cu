@@ -812,6 +812,166 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(2 * TC_BN));
 }
 
+// ------------------------------------------------- tcgen05 weight gradient
+// C[M x 256] += A^T B with A [K][M] and B [K][256] (bf16, K = positions, the
+// weight gradients of the 256-channel layers): both operands are MN-major, as
+// TMA brings them in (boxes of 64 channels x 64 positions, 128-byte swizzle).
+// A CTA accumulates 256 x 256 outputs (two M = 128 tiles, all 512 columns of
+// tensor memory) over its share of the positions and adds them to C with
+// 16-byte reductions; the positions are split so that the grid fills the SMs
+// once.  A may be the overlapping row view of the convolutions (row k + 1 starts
+// lda elements after row k): column m of row k is column m % lda of row
+// k + m / lda.  Roles, barriers and bounded waits as in gemm_ws_kernel.
+// Bound by the tiles' way from L2: 64 KB for 1024 clocks of MMA.  Measured (a
+// training step's 0.4M positions, M = 1280): about 1.15 -> 0.20 ms a layer
+// against the mma.sync form (0.27 TFLOP: 1.35 PFLOP/s).
+constexpr int WG_STAGES = 3, WG_BOX_BYTES = 64 * 64 * 2;
+constexpr int WG_STAGE_BYTES = 8 * WG_BOX_BYTES;           // A and B: 4 boxes each
+constexpr size_t WG_SMEM = (size_t)WG_STAGES * WG_STAGE_BYTES + 1024;
+// bf16 operands, both MN-major, fp32 accumulate, M = 128, N = 256
+constexpr uint32_t kIdescWg = kIdescBf16 | (1u << 15) | (1u << 16);
+
+// MN-major operand with the 128-byte swizzle: 64 elements of MN by 8 of K to a
+// 1024-byte atom; the next 64 elements of MN are one box further, the next 8
+// of K the next atom.
+__device__ __forceinline__ uint64_t umma_desc_mn128(uint32_t saddr) {
+  return umma_desc(saddr, WG_BOX_BYTES, 1024) | ((uint64_t)2 << 61);
+}
+
+__global__ void __launch_bounds__(WS_THREADS, 1)
+    gemm_wg_kernel(const __grid_constant__ CUtensorMap map_a,
+                   const __grid_constant__ CUtensorMap map_b, GemmArgs g, int a_row_len,
+                   int* err) {
+  extern __shared__ __align__(1024) unsigned char wgm[];
+  const uint32_t raw = smem_u32(wgm);
+  unsigned char* tiles = wgm + ((1024 - (raw & 1023)) & 1023);
+  __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], acc_full;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int abort_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.x * 256;
+  const int64_t kt_all = (g.K + 63) / 64;
+  const int64_t kt_per = (kt_all + gridDim.y - 1) / gridDim.y;
+  const int64_t kt_lo = (int64_t)blockIdx.y * kt_per;
+  const int ktiles = (int)max((int64_t)0, min(kt_per, kt_all - kt_lo));
+  if (ktiles == 0) return;                     // whole CTA
+
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&tmem_base_s)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (tid == 0) {
+    for (int s = 0; s < WG_STAGES; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&full[s])), "r"(1));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&empty[s])), "r"(1));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&acc_full)), "r"(1));
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  auto fail = [&]() {
+    abort_s = 1;
+    atomicExch(err, 1);
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      asm volatile("prefetch.tensormap [%0];" :: "l"(&map_a) : "memory");
+      asm volatile("prefetch.tensormap [%0];" :: "l"(&map_b) : "memory");
+      uint32_t loads[WG_STAGES] = {};
+      for (int kt = 0; kt < ktiles && !abort_s; ++kt) {
+        const int stage = kt % WG_STAGES;
+        if (!mbar_wait(smem_u32(&empty[stage]), ((kt / WG_STAGES) & 1u) ^ 1u)) { fail(); break; }
+        const uint32_t fb = smem_u32(&full[stage]);
+        mbar_expect_tx(fb, (uint32_t)WG_STAGE_BYTES);
+        const uint32_t a = smem_u32(tiles + stage * WG_STAGE_BYTES);
+        const int k0 = (int)((kt_lo + kt) * 64);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int m = m0 + 64 * j;
+          tma_load_2d(a + j * WG_BOX_BYTES, &map_a, m % a_row_len, k0 + m / a_row_len, fb);
+          tma_load_2d(a + (4 + j) * WG_BOX_BYTES, &map_b, 64 * j, k0, fb);
+        }
+        ++loads[stage];
+      }
+      // before exit every issued load has landed (see gemm_ws_kernel)
+      if (abort_s) {
+        for (int s2 = 0; s2 < WG_STAGES; ++s2)
+          if (loads[s2] > 0) mbar_wait(smem_u32(&full[s2]), (loads[s2] - 1) & 1u);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      for (int kt = 0; kt < ktiles && !abort_s; ++kt) {
+        const int stage = kt % WG_STAGES;
+        if (!mbar_wait(smem_u32(&full[stage]), (kt / WG_STAGES) & 1u)) { fail(); break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = smem_u32(tiles + stage * WG_STAGE_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const uint64_t db = umma_desc_mn128(a0 + 4 * WG_BOX_BYTES + ks * 2048);
+          const uint32_t accum = (kt > 0 || ks > 0) ? 1u : 0u;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint64_t da = umma_desc_mn128(a0 + i * 2 * WG_BOX_BYTES + ks * 2048);
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                :: "r"(tmem + (uint32_t)(i * 256)), "l"(da), "l"(db), "r"(kIdescWg), "r"(accum));
+          }
+        }
+        commit_to(smem_u32(&empty[stage]), 1u);
+      }
+      // covers every MMA issued, on the abort path too
+      commit_to(smem_u32(&acc_full), 1u);
+      if (!mbar_wait(smem_u32(&acc_full), 0)) fail();
+    }
+  } else {
+    const int e = warp - 2, q = warp & 3;
+    const bool done = mbar_wait(smem_u32(&acc_full), 0);
+    if (!done && lane == 0) fail();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int64_t m = m0 + (e >> 2) * 128 + q * 32 + lane;
+    if (done && !abort_s) {
+      float* crow = static_cast<float*>(g.C) + m * g.ldc;
+#pragma unroll 1
+      for (int c0 = 0; c0 < 256; c0 += 32) {
+        uint32_t v[32];
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((e >> 2) * 256 + c0);
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+            "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+              "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+              "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+              "=r"(v[31])
+            : "r"(taddr));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (m < g.M) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                         :: "l"(crow + c0 + j), "f"(__uint_as_float(v[j])),
+                            "f"(__uint_as_float(v[j + 1])), "f"(__uint_as_float(v[j + 2])),
+                            "f"(__uint_as_float(v[j + 3])) : "memory");
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512));
+}
+
 // ------------------------------------------------------------ elementwise
 // First convolution as a table.  Its input rows are class embeddings, so
 // the pre-activation of row p is b + sum_t T[t][cls[p-2+t]] with
@@ -951,6 +1111,83 @@ __global__ void embed_grad_kernel(const uint8_t* cls, int64_t P, const __nv_bflo
     const int64_t p = i / D;
     const int c = (int)(i - p * D), k = cls[p];
     if (k < 21) atomicAdd(dE + k * D + c, __bfloat162float(dX[i]));
+  }
+}
+
+// Gradients through the first convolution and the residue embedding.  The
+// layer's input rows are class embeddings, so both only need the sums of dZ by
+// class and tap, G[t][k] = sum of dZ[p] over the rows p with cls[p - 2 + t] == k:
+//   dW^T[(t, ci)] = sum_k E[k][ci] G[t][k],
+//   dE[k][ci]     = sum_t sum_co W[co][t][ci] G[t][k][co],
+// in place of a K = P weight-gradient GEMM over the embedded rows, a data-gradient
+// GEMM to 32 channels and a scatter of its rows by class.  Thread c of a
+// block owns channel c of a [5][21][256] table in shared memory (no two
+// threads share an entry), and adds the block's rows to it one after another;
+// bound by the 10 KB of shared memory a row reads and writes.  Measured on
+// a training step's 0.4M rows: about 1.1 ms for the four launches it replaces,
+// 0.33 for both kernels.
+constexpr int kClsTab = 5 * 21 * 256;
+__global__ void __launch_bounds__(256, 2) class_sum_kernel(const uint8_t* cls, int64_t P,
+                                                           const __nv_bfloat16* dZ, float* G) {
+  extern __shared__ float tab[];                 // [5][21][256]
+  const int c = threadIdx.x;
+  for (int i = c; i < kClsTab; i += 256) tab[i] = 0.f;
+  const int64_t rows = (P + gridDim.x - 1) / gridDim.x;
+  const int64_t p0 = (int64_t)blockIdx.x * rows, p1 = min(P, p0 + rows);
+  auto class_at = [&](int64_t q) { return q >= 0 && q < P ? (int)__ldg(cls + q) : 255; };
+  constexpr int B = 8;                           // rows in flight
+  int k[B + 4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) k[B + t] = class_at(p0 - 2 + t);
+  for (int64_t p = p0; p < p1; p += B) {
+    float z[B];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) k[t] = k[B + t];
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      z[i] = p + i < p1 ? __bfloat162float(dZ[(p + i) * 256 + c]) : 0.f;
+      k[4 + i] = class_at(p + 2 + i);
+    }
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      // the five taps' entries are distinct: all read before any is written
+      float v[5];
+#pragma unroll
+      for (int t = 0; t < 5; ++t) {
+        v[t] = 0.f;
+        if (k[i + t] < 21) v[t] = tab[(t * 21 + k[i + t]) * 256 + c];
+      }
+#pragma unroll
+      for (int t = 0; t < 5; ++t)
+        if (k[i + t] < 21) tab[(t * 21 + k[i + t]) * 256 + c] = v[t] + z[i];
+    }
+  }
+  for (int i = c; i < kClsTab; i += 256)
+    if (tab[i] != 0.f) atomicAdd(G + i, tab[i]);
+}
+
+// Blocks 0 .. 5 * cin - 1: row (t, ci) of dW^T; the next 21: row k of dE.
+__global__ void __launch_bounds__(256) conv1_grad_kernel(const float* G, const __nv_bfloat16* E,
+                                                         const __nv_bfloat16* Wf, int cin,
+                                                         float* dWT, float* dE) {
+  const int c = threadIdx.x;
+  if ((int)blockIdx.x < 5 * cin) {
+    const int t = blockIdx.x / cin, ci = blockIdx.x - t * cin;
+    float acc = 0.f;
+    for (int k = 0; k < 21; ++k)
+      acc = fmaf(__bfloat162float(E[k * cin + ci]), G[(t * 21 + k) * 256 + c], acc);
+    dWT[(int64_t)blockIdx.x * 256 + c] += acc;
+    return;
+  }
+  const int k = blockIdx.x - 5 * cin, warp = c >> 5, lane = c & 31;
+  for (int ci = warp; ci < cin; ci += 8) {       // a warp per input channel
+    float acc = 0.f;
+    for (int t = 0; t < 5; ++t)
+      for (int co = lane; co < 256; co += 32)    // Wf[ci][4 - t][co] = W[co][t][ci]
+        acc = fmaf(__bfloat162float(Wf[((int64_t)ci * 5 + (4 - t)) * 256 + co]),
+                   G[(t * 21 + k) * 256 + co], acc);
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) dE[k * cin + ci] += acc;
   }
 }
 
@@ -1113,14 +1350,24 @@ __global__ void pool_backward_kernel(const float* emb, const float* dE, const fl
   }
 }
 
-// db[c] += sum over rows of dZ[p][c] (block: 256 columns x a row range)
+// db[c] += sum over rows of dZ[p][c] (block: 256 columns x a row range).
+// D = 256 (16-byte aligned dZ) reads 16 bytes a lane, a row a warp (0.4M rows:
+// 60 -> 37 us a layer; reading them once takes 31).
 __global__ void bias_grad_kernel(const __nv_bfloat16* dZ, int64_t P, int D, float* db) {
-  const int c = threadIdx.x + blockIdx.y * blockDim.x;
-  if (c >= D) return;
   const int64_t rows = (P + gridDim.x - 1) / gridDim.x;
   const int64_t p0 = (int64_t)blockIdx.x * rows, p1 = min(P, p0 + rows);
+  __shared__ float part[8][256];
+  const int c = threadIdx.x + blockIdx.y * blockDim.x;
   float acc = 0.f;
-  for (int64_t p = p0; p < p1; ++p) acc += __bfloat162float(dZ[p * D + c]);
+  if (D == 256 && (reinterpret_cast<uintptr_t>(dZ) & 15) == 0) {
+    sum_rows256(dZ + p0 * 256, (int)max((int64_t)0, p1 - p0), c >> 5, 8, c & 31, part);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) acc += part[w][c];
+  } else {
+    if (c >= D) return;
+    for (int64_t p = p0; p < p1; ++p) acc += __bfloat162float(dZ[p * D + c]);
+  }
   atomicAdd(db + c, acc);
 }
 
@@ -1725,6 +1972,35 @@ int launch_tc_ws(const GemmArgs& g, cudaStream_t stream) {
   return status_of(cudaGetLastError());
 }
 
+// The MN-major kernel applies when 64-column boxes of A stay inside its rows
+// (a plain matrix, or an overlapping view with lda % 64 == 0) and C takes
+// 16-byte reductions.
+static bool wg_applies(const GemmArgs& g) {
+  return g.N == 256 && g.K >= 64 && (g.lda >= g.M || g.lda % 64 == 0) && g.ldb >= 256 &&
+         g.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
+         g.M <= 256 * 65535 && g.K + g.M / std::max<int64_t>(1, g.lda) < INT32_MAX - 256;
+}
+
+static int launch_wg(const GemmArgs& g, cudaStream_t stream) {
+  int* err = tc_error_flag();
+  if (!err) return SSEQS_ERR_CUDA;
+  const bool plain = g.lda >= g.M;
+  CUtensorMap ma, mb;
+  if (!make_map(&ma, g.A, plain ? g.M : g.lda, g.K + (plain ? 0 : (g.M - 1) / g.lda), g.lda, 64) ||
+      !make_map(&mb, g.B, 256, g.K, g.ldb, 64))
+    return SSEQS_ERR_CUDA;
+  if (cudaFuncSetAttribute((const void*)gemm_wg_kernel,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM) != cudaSuccess)
+    return SSEQS_ERR_CUDA;
+  const int mt = (int)((g.M + 255) / 256);
+  const int splits = (int)std::max<int64_t>(
+      1, std::min<int64_t>(device_sm_count() / mt, (g.K + 63) / 64));
+  const int row_len = plain ? 256 * mt + 256 : (int)g.lda;      // > every m when plain
+  { gemm_wg_kernel<<<dim3(mt, splits), WS_THREADS, WG_SMEM, stream>>>(ma, mb, g, row_len, err);
+    count_launches(1); }
+  return status_of(cudaGetLastError());
+}
+
 // 1 = use the tcgen05 kernel where it applies (default), 0 = mma.sync only.
 extern "C" int sseqs_gemm_set_tensor_path(int tcgen05) {
   g_tc_enabled = tcgen05 != 0;
@@ -1768,6 +2044,7 @@ extern "C" int sseqs_gemm_bf16(int a_t, int b_t, int epilogue, int64_t M, int64_
     // split K so that the grid covers every SM twice (C holds the sum of
     // the partial products; the caller zeroes it)
     if (a_t != 1 || b_t != 1) return SSEQS_ERR_UNSUPPORTED;
+    if (g_tc_enabled && wg_applies(g)) return launch_wg(g, stream);
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int64_t want = (2 * (int64_t)device_sm_count() + tiles - 1) / tiles;
     const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(want, K / BK));
@@ -1863,6 +2140,27 @@ extern "C" int sseqs_embed_grad(const uint8_t* cls, int64_t P, const void* dX, i
   if (P == 0) return SSEQS_OK;
   { embed_grad_kernel<<<grid_for(P * D, 256), 256, 0, stream>>>(
         cls, P, static_cast<const __nv_bfloat16*>(dX), D, dE);
+    count_launches(1); }
+  return status_of(cudaGetLastError());
+}
+
+extern "C" int sseqs_embed_conv1_grad(const uint8_t* cls, int64_t P, const void* dZ, int D,
+                                      const void* E, int cin, const void* Wf, float* G,
+                                      float* dWT, float* dE, cudaStream_t stream) {
+  if (P < 0 || D != 256 || cin < 1 || cin > 4096) return SSEQS_ERR_ARG;
+  if (P == 0) return SSEQS_OK;
+  if (!cls || !dZ || !E || !Wf || !G || !dWT || !dE) return SSEQS_ERR_ARG;
+  const size_t smem = sizeof(float) * kClsTab;
+  if (cudaFuncSetAttribute((const void*)class_sum_kernel,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return SSEQS_ERR_CUDA;
+  if (cudaMemsetAsync(G, 0, smem, stream) != cudaSuccess) return SSEQS_ERR_CUDA;
+  const int grid = (int)std::min<int64_t>((P + 63) / 64, (int64_t)device_sm_count() * 2);
+  { class_sum_kernel<<<grid, 256, smem, stream>>>(cls, P, static_cast<const __nv_bfloat16*>(dZ), G);
+    count_launches(1); }
+  { conv1_grad_kernel<<<5 * cin + 21, 256, 0, stream>>>(
+        G, static_cast<const __nv_bfloat16*>(E), static_cast<const __nv_bfloat16*>(Wf), cin, dWT,
+        dE);
     count_launches(1); }
   return status_of(cudaGetLastError());
 }

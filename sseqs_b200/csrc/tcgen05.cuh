@@ -56,7 +56,6 @@ __device__ __forceinline__ void commit_to(uint32_t mbar, uint32_t leader) {
   if (leader)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  :: "r"(mbar) : "memory");
-  __syncwarp();
 }
 
 // Shared-memory matrix descriptor: start, leading (K) and stride (MN)

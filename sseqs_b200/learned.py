@@ -101,14 +101,11 @@ class _Buffers:
     def __init__(self, rows: int, train: bool, dev):
         self.rows = rows
         z = lambda c: torch.zeros((rows + 4, c), dtype=torch.bfloat16, device=dev)
-        # inference keeps two layer outputs (alternating), no embedded rows
-        # and no pre-activations
-        self.X0 = z(E) if train else None
+        # inference keeps two layer outputs (alternating) and no pre-activations
         self.Y = [z(D) for _ in range(4 if train else 2)]
         self.Z = [z(D) for _ in range(4)] if train else None
         self.dZ = [z(D) for _ in range(4)] if train else None
         self.G = [z(D) for _ in range(4)] if train else None
-        self.dX0 = z(E) if train else None
 
 
 def _base(buf: torch.Tensor) -> int:
@@ -178,9 +175,6 @@ class Embedder:
         bufs = self._buffers(lay.P, train)
         P = lay.P
         L = lib()
-        if train:    # the backward pass reads the embedded rows
-            check(L.sseqs_embed_lookup(ptr(lay.cls), P, ptr(self.emb_b), E, _base(bufs.X0),
-                                       stream_ptr()), "embed_lookup")
         # layer 1 from its table (a K = 160 GEMM otherwise); the pre-activations
         # Z are kept for the backward pass only
         check(L.sseqs_embed_conv1_table(ptr(lay.cls), P, ptr(self.T1), ptr(self.b[0]),
@@ -221,14 +215,21 @@ class Embedder:
                                     _base(bufs.dZ[3]), _base(bufs.G[3]), stream_ptr()),
               "pool_backward")
         grads = {"W": [None] * 4, "b": [None] * 4}
+        dEmb = torch.zeros((NCLS, E), dtype=torch.float32, device=self.device)
         for l in range(3, -1, -1):
             cin = self.cin[l]
-            prev = bufs.Y[l - 1] if l > 0 else bufs.X0
             dZ = bufs.dZ[l]
             dWT = torch.zeros((5 * cin, D), dtype=torch.float32, device=self.device)
-            # dW^T = im2col(prev)^T . dZ over the P rows (split over positions)
-            _gemm(1, 1, _EPI_F32_ADD, 5 * cin, D, P, prev.data_ptr(), cin, _base(dZ), D,
-                  dWT.data_ptr(), D)
+            if l > 0:
+                # dW^T = im2col(prev)^T . dZ over the P rows (split over positions)
+                _gemm(1, 1, _EPI_F32_ADD, 5 * cin, D, P, bufs.Y[l - 1].data_ptr(), cin, _base(dZ),
+                      D, dWT.data_ptr(), D)
+            else:
+                # layer 1 and the embedding, from the sums of dZ by class and tap
+                sums = torch.empty(5 * NCLS * D, dtype=torch.float32, device=self.device)
+                check(L.sseqs_embed_conv1_grad(ptr(lay.cls), P, _base(dZ), D, ptr(self.emb_b),
+                                               cin, ptr(self.Wf[0]), ptr(sums), ptr(dWT),
+                                               ptr(dEmb), stream_ptr()), "conv1_grad")
             db = torch.zeros(D, dtype=torch.float32, device=self.device)
             check(L.sseqs_bias_grad(_base(dZ), P, D, ptr(db), stream_ptr()), "bias_grad")
             grads["W"][l], grads["b"][l] = dWT, db
@@ -243,12 +244,6 @@ class Embedder:
                 _gemm(0, 0, _EPI_GELU_GRAD, P, cin, 5 * D, dZ.data_ptr(), D,
                       self.Wf[l].data_ptr(), 5 * D, _base(bufs.dZ[l - 1]), cin, None, None,
                       _base(bufs.Z[l - 1]), lay.mask)
-            else:
-                _gemm(0, 0, _EPI_BF16, P, cin, 5 * D, dZ.data_ptr(), D, self.Wf[0].data_ptr(),
-                      5 * D, _base(bufs.dX0), cin, None, None, None, lay.mask)
-        dEmb = torch.zeros((NCLS, E), dtype=torch.float32, device=self.device)
-        check(L.sseqs_embed_grad(ptr(lay.cls), P, _base(bufs.dX0), E, ptr(dEmb), stream_ptr()),
-              "embed_grad")
         grads["emb"] = dEmb
         return grads
 
