@@ -184,7 +184,7 @@ int sseqs_topk(const void* keys, int key_type, int64_t n, int64_t k, int32_t* ou
  * caching pool, a server's fixed budget) and may not take memory behind its
  * back, or a latency-critical caller that cannot afford the stalls that
  * cudaMalloc / cudaFree can cause.  The caller passes keys and out_idx only;
- * the scratch is a fixed array inside this library (about 66 KB per GPU that
+ * the scratch is a fixed array inside this library (about 74 KB per GPU that
  * loads the library, held until the process exits), so n is limited to
  * SSEQS_TOPK_STATIC_MAX_N keys -- larger n returns SSEQS_ERR_CAPACITY.  The
  * first call on a device looks up that array's device address (with the

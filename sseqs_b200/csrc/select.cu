@@ -11,9 +11,9 @@
 // pass 1 counts selected items per tile, pass 2 turns the counts into
 // exclusive offsets (one block), pass 3 re-evaluates the predicate and writes
 // each selected item at offset + rank-in-tile (a block-wide scan), so outputs
-// keep input order.  Top-k finds the exact k-th largest key with four
-// 8-bit radix passes (shared-memory histograms merged with 256 global atomics
-// per block) before compacting.
+// keep input order.  Top-k finds the exact k-th largest key with radix passes
+// of up to 11 bits (shared-memory histograms; the last block of a pass picks the
+// digit) before compacting; up to kSmallN keys take one block and one launch.
 #include <algorithm>
 #include <mutex>
 
@@ -26,16 +26,22 @@ constexpr int kSelThreads = 256;
 constexpr int kItems = 16;                      // items per thread and tile
 constexpr int kTile = kSelThreads * kItems;     // 4096
 
+constexpr int kDigitBits = 11, kDigits = 1 << kDigitBits;
+
+// All zero at the start of a call.
 struct TopkCtl {
   uint32_t prefix;     // key bits fixed so far
   uint32_t mask;       // which bits of prefix are fixed
-  int64_t kleft;       // elements still to take at or below the prefix
-  uint32_t hist[256];
+  int64_t taken;       // elements above the prefix, which are all taken
+  uint32_t done;       // blocks of the running pass that have finished
+  uint32_t hist[kDigits];
 };
 
 // Block-wide exclusive scan of one int64 per thread; returns the total.
+template <int THREADS = kSelThreads>
 __device__ __forceinline__ int64_t block_exclusive_scan(int64_t v, int64_t* out_excl) {
-  __shared__ int64_t warp_sums[kSelThreads / 32];
+  static_assert(THREADS % 32 == 0 && THREADS <= 1024, "at most 32 warps");
+  __shared__ int64_t warp_sums[THREADS / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int64_t x = v;
 #pragma unroll
@@ -46,17 +52,17 @@ __device__ __forceinline__ int64_t block_exclusive_scan(int64_t v, int64_t* out_
   if (lane == 31) warp_sums[wid] = x;
   __syncthreads();
   if (wid == 0) {
-    int64_t s = (lane < kSelThreads / 32) ? warp_sums[lane] : 0;
+    int64_t s = (lane < THREADS / 32) ? warp_sums[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int64_t y = __shfl_up_sync(0xffffffffu, s, o);
       if (lane >= o) s += y;
     }
-    if (lane < kSelThreads / 32) warp_sums[lane] = s;
+    if (lane < THREADS / 32) warp_sums[lane] = s;
   }
   __syncthreads();
   const int64_t before = (wid == 0 ? 0 : warp_sums[wid - 1]) + x - v;
-  const int64_t total = warp_sums[kSelThreads / 32 - 1];
+  const int64_t total = warp_sums[THREADS / 32 - 1];
   __syncthreads();
   *out_excl = before;
   return total;
@@ -159,62 +165,137 @@ __device__ __forceinline__ uint32_t key_of(const void* keys, int64_t i) {
   }
 }
 
-__global__ void topk_init_kernel(TopkCtl* ctl, int64_t k) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) ctl->hist[i] = 0;
-  if (threadIdx.x == 0) {
-    ctl->prefix = 0;
-    ctl->mask = 0;
-    ctl->kleft = k;
-  }
-}
-
-template <int KT>
-__global__ void __launch_bounds__(kSelThreads)
-    topk_hist_kernel(const void* keys, int64_t n, TopkCtl* ctl, int shift) {
-  __shared__ uint32_t h[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  const uint32_t prefix = ctl->prefix, mask = ctl->mask;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t k = key_of<KT>(keys, i);
-    if ((k & mask) == prefix) atomicAdd(&h[(k >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 256; i += blockDim.x)
-    if (h[i]) atomicAdd(&ctl->hist[i], h[i]);
-}
-
-__global__ void topk_pick_kernel(TopkCtl* ctl, int shift) {
-  if (threadIdx.x == 0) {
-    int64_t above = 0;
-    int d = 255;
-    for (; d > 0; --d) {
-      const int64_t c = ctl->hist[d];
-      if (above + c >= ctl->kleft) break;
-      above += c;
+// The digit that holds the k-th largest of the keys a histogram counts, and how
+// many keys lie in higher digits; found by the whole block, each
+// thread holding kDigits / THREADS digits from the highest down.
+struct Pick {
+  int digit;
+  int64_t above;
+};
+template <int THREADS = kSelThreads, class Hist>
+__device__ __forceinline__ Pick pick_digit(Hist count, int64_t k) {
+  constexpr int PER = kDigits / THREADS;
+  __shared__ int digit_s;
+  __shared__ int64_t above_s;
+  const int top = kDigits - 1 - (int)threadIdx.x * PER;
+  int64_t c[PER], sum = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) { c[i] = count(top - i); sum += c[i]; }
+  int64_t before;
+  block_exclusive_scan<THREADS>(sum, &before);
+  if (before < k && k <= before + sum) {      // one thread: 1 <= k <= all keys
+    int64_t above = before;
+    int d = top;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      if (top - i == d && above + c[i] < k) { above += c[i]; --d; }
     }
-    ctl->prefix |= (uint32_t)d << shift;
-    ctl->mask |= 255u << shift;
-    ctl->kleft -= above;
+    digit_s = d;
+    above_s = above;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) ctl->hist[i] = 0;
+  const Pick p{digit_s, above_s};
+  __syncthreads();
+  return p;
 }
 
+// Adds one to bin `d` for every lane with `live`; a warp whose live lanes all
+// have the same digit (the high digits of scores) adds once.
+__device__ __forceinline__ void count_digit(uint32_t* h, uint32_t d, bool live) {
+  const unsigned m = __ballot_sync(0xffffffffu, live);
+  if (m == 0) return;
+  const int src = __ffs(m) - 1;
+  const uint32_t first = __shfl_sync(0xffffffffu, d, src);
+  if (__all_sync(0xffffffffu, !live || d == first)) {
+    if ((int)(threadIdx.x & 31) == src) atomicAdd(&h[first], (uint32_t)__popc(m));
+  } else if (live) {
+    atomicAdd(&h[d], 1u);
+  }
+}
+
+// True in every thread of the last block to get here; the other blocks' writes
+// are visible to it.
+__device__ __forceinline__ bool last_block(uint32_t* done) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  __threadfence();
+  return last;
+}
+
+constexpr int kHistItems = 8, kHistTile = kSelThreads * kHistItems;
+
+// One radix pass: counts digit [shift, shift + bits) of the keys that agree
+// with the prefix; the last block extends the prefix by the digit of the k-th largest
+// key and clears the counters (one launch a pass: a pass's pick as a launch of its own,
+// one thread walking the bins, took 12 us).
 template <int KT>
 __global__ void __launch_bounds__(kSelThreads)
-    topk_count_kernel(const void* keys, int64_t n, const TopkCtl* ctl, int64_t* cnt_gt, int64_t* cnt_eq) {
+    topk_hist_kernel(const void* keys, int64_t n, int64_t k, TopkCtl* ctl, int shift, int bits) {
+  __shared__ uint32_t h[kDigits];
+  for (int i = threadIdx.x; i < kDigits; i += blockDim.x) h[i] = 0;
+  __syncthreads();
+  const uint32_t prefix = ctl->prefix, mask = ctl->mask, dm = (1u << bits) - 1u;
+  // kHistItems keys a thread are read before any is counted
+  const int64_t step = (int64_t)gridDim.x * kHistTile;
+  for (int64_t b = (int64_t)blockIdx.x * kHistTile; b < n; b += step) {
+    uint32_t key[kHistItems];
+#pragma unroll
+    for (int j = 0; j < kHistItems; ++j) {
+      const int64_t i = b + j * kSelThreads + threadIdx.x;
+      key[j] = i < n ? key_of<KT>(keys, i) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kHistItems; ++j) {
+      const int64_t i = b + j * kSelThreads + threadIdx.x;
+      count_digit(h, (key[j] >> shift) & dm, i < n && (key[j] & mask) == prefix);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kDigits; i += blockDim.x)
+    if (h[i]) atomicAdd(&ctl->hist[i], h[i]);
+  if (!last_block(&ctl->done)) return;
+  const Pick p = pick_digit([&](int d) { return (int64_t)__ldcg(&ctl->hist[d]); },
+                            k - ctl->taken);
+  for (int i = threadIdx.x; i < kDigits; i += blockDim.x) ctl->hist[i] = 0;
+  if (threadIdx.x == 0) {
+    ctl->prefix = prefix | ((uint32_t)p.digit << shift);
+    ctl->mask = mask | (dm << shift);
+    ctl->taken += p.above;
+    ctl->done = 0;
+  }
+}
+
+// Exclusive scan of cnt[0..m) in place by one block, values other blocks wrote.
+__device__ __forceinline__ void scan_tiles(int64_t* cnt, int64_t m) {
+  int64_t carry = 0;
+  for (int64_t base = 0; base < m; base += kSelThreads) {
+    const int64_t i = base + threadIdx.x;
+    const int64_t v = i < m ? __ldcg(cnt + i) : 0;
+    int64_t ex;
+    const int64_t tot = block_exclusive_scan(v, &ex);
+    if (i < m) cnt[i] = carry + ex;
+    carry += tot;
+  }
+}
+
+// Keys above and at the k-th largest, per tile; the last block turns both
+// counts into offsets.
+template <int KT>
+__global__ void __launch_bounds__(kSelThreads)
+    topk_count_kernel(const void* keys, int64_t n, TopkCtl* ctl, int64_t* cnt_gt, int64_t* cnt_eq) {
   const uint32_t T = ctl->prefix;
   const int64_t ntile = (n + kTile - 1) / kTile;
   __shared__ int wg[kSelThreads / 32], we[kSelThreads / 32];
   for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    const int64_t b = tile * kTile + (int64_t)threadIdx.x * kItems;
     int g = 0, e = 0;
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
-      if (b + i < n) {
-        const uint32_t k = key_of<KT>(keys, b + i);
+      const int64_t x = tile * kTile + (int64_t)i * kSelThreads + threadIdx.x;
+      if (x < n) {
+        const uint32_t k = key_of<KT>(keys, x);
         g += k > T;
         e += k == T;
       }
@@ -231,14 +312,17 @@ __global__ void __launch_bounds__(kSelThreads)
     }
     __syncthreads();
   }
+  if (!last_block(&ctl->done)) return;
+  scan_tiles(cnt_gt, ntile);
+  scan_tiles(cnt_eq, ntile);
 }
 
 template <int KT>
 __global__ void __launch_bounds__(kSelThreads)
-    topk_scatter_kernel(const void* keys, int64_t n, const TopkCtl* ctl, const int64_t* off_gt,
-                        const int64_t* off_eq, int32_t* out_idx) {
+    topk_scatter_kernel(const void* keys, int64_t n, int64_t k, const TopkCtl* ctl,
+                        const int64_t* off_gt, const int64_t* off_eq, int32_t* out_idx) {
   const uint32_t T = ctl->prefix;
-  const int64_t kleft = ctl->kleft;
+  const int64_t kleft = k - ctl->taken;          // keys equal to T that are taken
   const int64_t ntile = (n + kTile - 1) / kTile;
   for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
     const int64_t b = tile * kTile + (int64_t)threadIdx.x * kItems;
@@ -247,15 +331,15 @@ __global__ void __launch_bounds__(kSelThreads)
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       if (b + i < n) {
-        const uint32_t k = key_of<KT>(keys, b + i);
-        if (k > T) { gb |= 1u << i; ++g; }
-        else if (k == T) { eb |= 1u << i; ++e; }
+        const uint32_t key = key_of<KT>(keys, b + i);
+        if (key > T) { gb |= 1u << i; ++g; }
+        else if (key == T) { eb |= 1u << i; ++e; }
       }
     }
-    int64_t gx, ex;
-    block_exclusive_scan(g, &gx);
-    block_exclusive_scan(e, &ex);
-    int64_t G = off_gt[tile] + gx, E = off_eq[tile] + ex;
+    // both counts in one scan
+    int64_t x;
+    block_exclusive_scan(((int64_t)g << 32) | e, &x);
+    int64_t G = off_gt[tile] + (x >> 32), E = off_eq[tile] + (x & 0xffffffff);
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       const bool isg = gb & (1u << i), ise = eb & (1u << i);
@@ -263,6 +347,60 @@ __global__ void __launch_bounds__(kSelThreads)
       G += isg;
       E += ise;
     }
+  }
+}
+
+// The whole selection by one block, for up to kSmallN keys, held in registers
+// (thread t: keys t * per ..): the candidate lists of a search at the
+// default settings hold some hundred to some thousand.  1400 keys: 14 launches
+// and 75 us before, one of 9 us; the tiled form takes 6 and about 28 us at 100k.
+constexpr int kSmallThreads = 1024, kSmallItems = 16, kSmallN = kSmallThreads * kSmallItems;
+template <int KT>
+__global__ void __launch_bounds__(kSmallThreads)
+    topk_small_kernel(const void* keys, int n, int64_t k, int32_t* out_idx) {
+  __shared__ uint32_t h[kDigits];
+  const int per = (n + kSmallThreads - 1) / kSmallThreads, first = (int)threadIdx.x * per;
+  uint32_t key[kSmallItems];
+#pragma unroll
+  for (int i = 0; i < kSmallItems; ++i)
+    key[i] = i < per && first + i < n ? key_of<KT>(keys, first + i) : 0u;
+  uint32_t prefix = 0, mask = 0;
+  int64_t taken = 0;
+  constexpr int kPasses = KT == 0 ? 3 : 2;
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) {
+    const int shift = KT == 0 ? (p == 0 ? 21 : p == 1 ? 10 : 0) : (p == 0 ? 8 : 0);
+    const uint32_t dm = KT == 0 ? (p < 2 ? 2047u : 1023u) : 255u;
+    for (int i = threadIdx.x; i < kDigits; i += kSmallThreads) h[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i)
+      if (i < per)
+        count_digit(h, (key[i] >> shift) & dm, first + i < n && (key[i] & mask) == prefix);
+    __syncthreads();
+    const Pick pk = pick_digit<kSmallThreads>([&](int d) { return (int64_t)h[d]; }, k - taken);
+    prefix |= (uint32_t)pk.digit << shift;
+    mask |= dm << shift;
+    taken += pk.above;
+  }
+  const int64_t kleft = k - taken;
+  int g = 0, e = 0;
+#pragma unroll
+  for (int i = 0; i < kSmallItems; ++i) {
+    const bool live = i < per && first + i < n;
+    g += live && key[i] > prefix;
+    e += live && key[i] == prefix;
+  }
+  int64_t x;
+  block_exclusive_scan<kSmallThreads>(((int64_t)g << 32) | e, &x);
+  int64_t G = x >> 32, E = x & 0xffffffff;
+#pragma unroll
+  for (int i = 0; i < kSmallItems; ++i) {
+    const bool live = i < per && first + i < n;
+    const bool isg = live && key[i] > prefix, ise = live && key[i] == prefix;
+    if (isg || (ise && E < kleft)) out_idx[G + min(E, kleft)] = first + i;
+    G += isg;
+    E += ise;
   }
 }
 
@@ -438,6 +576,32 @@ extern "C" size_t sseqs_topk_workspace_bytes(int64_t n) {
   return align256(sizeof(TopkCtl)) + 2 * align256(sizeof(int64_t) * (size_t)std::max<int64_t>(tiles, 1));
 }
 
+namespace {
+// Top-k with the control block and per-tile counters the caller provides
+// (checked arguments, 0 < k <= n).
+template <int KT>
+int run_topk(const void* keys, int64_t n, int64_t k, int32_t* out_idx, TopkCtl* ctl, int64_t* cg,
+             int64_t* ce, cudaStream_t stream) {
+  if (n <= kSmallN) {
+    { topk_small_kernel<KT><<<1, kSmallThreads, 0, stream>>>(keys, (int)n, k, out_idx); count_launches(1); }
+    return status_of(cudaGetLastError());
+  }
+  if (cudaMemsetAsync(ctl, 0, sizeof(TopkCtl), stream) != cudaSuccess) return SSEQS_ERR_CUDA;
+  const int hgrid = (int)std::min<int64_t>((n + kHistTile - 1) / kHistTile,
+                                           (int64_t)device_sm_count() * 4);
+  const int shifts[3] = {KT == 0 ? 21 : 8, KT == 0 ? 10 : 0, 0};
+  const int bits[3] = {KT == 0 ? 11 : 8, KT == 0 ? 11 : 8, 10};
+  for (int p = 0; p < (KT == 0 ? 3 : 2); ++p)
+    { topk_hist_kernel<KT><<<hgrid, kSelThreads, 0, stream>>>(keys, n, k, ctl, shifts[p], bits[p]);
+      count_launches(1); }
+  const int grid = grid_for(n);
+  { topk_count_kernel<KT><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce); count_launches(1); }
+  { topk_scatter_kernel<KT><<<grid, kSelThreads, 0, stream>>>(keys, n, k, ctl, cg, ce, out_idx);
+    count_launches(1); }
+  return status_of(cudaGetLastError());
+}
+}  // namespace
+
 extern "C" int sseqs_topk(const void* keys, int key_type, int64_t n, int64_t k, int32_t* out_idx,
                           void* workspace, size_t ws_bytes, cudaStream_t stream) {
   if (n < 0 || k < 0 || k > n || (key_type != 0 && key_type != 1)) return SSEQS_ERR_ARG;
@@ -456,25 +620,8 @@ extern "C" int sseqs_topk(const void* keys, int key_type, int64_t n, int64_t k, 
   int64_t* cg = reinterpret_cast<int64_t*>(ws);
   ws += align256(sizeof(int64_t) * (size_t)tiles);
   int64_t* ce = reinterpret_cast<int64_t*>(ws);
-  const int grid = grid_for(n);
-  const int hgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kSelThreads - 1) / kSelThreads,
-                                                                (int64_t)device_sm_count() * 4));
-  { topk_init_kernel<<<1, 256, 0, stream>>>(ctl, k); count_launches(1); }
-  const int first_shift = key_type == 0 ? 24 : 8;
-  for (int shift = first_shift; shift >= 0; shift -= 8) {
-    if (key_type == 0)
-      { topk_hist_kernel<0><<<hgrid, kSelThreads, 0, stream>>>(keys, n, ctl, shift); count_launches(1); }
-    else
-      { topk_hist_kernel<1><<<hgrid, kSelThreads, 0, stream>>>(keys, n, ctl, shift); count_launches(1); }
-    { topk_pick_kernel<<<1, 256, 0, stream>>>(ctl, shift); count_launches(1); }
-  }
-  if (key_type == 0) { topk_count_kernel<0><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce); count_launches(1); }
-  else { topk_count_kernel<1><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce); count_launches(1); }
-  { scan_counts_kernel<<<1, kSelThreads, 0, stream>>>(cg, tiles, nullptr); count_launches(1); }
-  { scan_counts_kernel<<<1, kSelThreads, 0, stream>>>(ce, tiles, nullptr); count_launches(1); }
-  if (key_type == 0) { topk_scatter_kernel<0><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce, out_idx); count_launches(1); }
-  else { topk_scatter_kernel<1><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce, out_idx); count_launches(1); }
-  return status_of(cudaGetLastError());
+  return key_type == 0 ? run_topk<0>(keys, n, k, out_idx, ctl, cg, ce, stream)
+                       : run_topk<1>(keys, n, k, out_idx, ctl, cg, ce, stream);
 }
 
 // ------------------------------------------------------------ hit windows
@@ -535,7 +682,7 @@ extern "C" int sseqs_pack_segments(const uint64_t* bases, const int32_t* part, c
 // ------------------------------------------------ top-k without allocation
 // Scratch of sseqs_topk_static: the same control block and per-tile counters
 // as sseqs_topk's workspace, in a fixed array that every GPU loading this
-// library holds until the process exits (about 66 KB).  Host code may not
+// library holds until the process exits (about 74 KB).  Host code may not
 // pass this symbol to a kernel (on the host it names a stand-in, not device
 // memory); it uses the device address fetched below.
 namespace {
@@ -579,30 +726,12 @@ extern "C" int sseqs_topk_static(const void* keys, int key_type, int64_t n, int6
   unsigned char* base = nullptr;
   const int st = static_topk_scratch(&base);
   if (st != SSEQS_OK) return st;
-  // The control block is rewritten by topk_init_kernel at the start of every
-  // call, and every counter slot a call reads is written earlier in the same
-  // call, so nothing left over from a previous call is read.
+  // The control block is cleared at the start of every call, and every counter
+  // slot a call reads is written earlier in the same call, so nothing left
+  // over from a previous call is read.
   TopkCtl* ctl = reinterpret_cast<TopkCtl*>(base);
   int64_t* cg = reinterpret_cast<int64_t*>(base + kStaticCtlBytes);
   int64_t* ce = cg + kStaticTopkTiles;
-  const int64_t tiles = (n + kTile - 1) / kTile;
-  const int grid = grid_for(n);
-  const int hgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kSelThreads - 1) / kSelThreads,
-                                                                (int64_t)device_sm_count() * 4));
-  { topk_init_kernel<<<1, 256, 0, stream>>>(ctl, k); count_launches(1); }
-  const int first_shift = key_type == 0 ? 24 : 8;
-  for (int shift = first_shift; shift >= 0; shift -= 8) {
-    if (key_type == 0)
-      { topk_hist_kernel<0><<<hgrid, kSelThreads, 0, stream>>>(keys, n, ctl, shift); count_launches(1); }
-    else
-      { topk_hist_kernel<1><<<hgrid, kSelThreads, 0, stream>>>(keys, n, ctl, shift); count_launches(1); }
-    { topk_pick_kernel<<<1, 256, 0, stream>>>(ctl, shift); count_launches(1); }
-  }
-  if (key_type == 0) { topk_count_kernel<0><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce); count_launches(1); }
-  else { topk_count_kernel<1><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce); count_launches(1); }
-  { scan_counts_kernel<<<1, kSelThreads, 0, stream>>>(cg, tiles, nullptr); count_launches(1); }
-  { scan_counts_kernel<<<1, kSelThreads, 0, stream>>>(ce, tiles, nullptr); count_launches(1); }
-  if (key_type == 0) { topk_scatter_kernel<0><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce, out_idx); count_launches(1); }
-  else { topk_scatter_kernel<1><<<grid, kSelThreads, 0, stream>>>(keys, n, ctl, cg, ce, out_idx); count_launches(1); }
-  return status_of(cudaGetLastError());
+  return key_type == 0 ? run_topk<0>(keys, n, k, out_idx, ctl, cg, ce, stream)
+                       : run_topk<1>(keys, n, k, out_idx, ctl, cg, ce, stream);
 }
