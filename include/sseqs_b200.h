@@ -50,6 +50,26 @@ int sseqs_max_query_len(void);
  * the stream that starts at packed[lo_bytes]. */
 int sseqs_xbit_decompress(const uint8_t* packed, uint8_t* out, int64_t n_syms,
                           int64_t lo_bytes, cudaStream_t stream);
+/* Decodes as sseqs_xbit_decompress and notes the '@' symbols on the way:
+ * info[0] = index of the last other symbol (-1: none), info[1] = number of '@'
+ * (device, int64[2]).  The workspace then holds what sseqs_decode_scan_delims
+ * needs to write the positions of the first n_delims of them (each at most
+ * INT32_MAX), increasing, to out_pos. */
+size_t sseqs_decode_scan_workspace_bytes(int64_t n_syms);
+int sseqs_decode_scan(const uint8_t* packed, uint8_t* out, int64_t n_syms, int64_t lo_bytes,
+                      int64_t* info, void* workspace, size_t ws_bytes, cudaStream_t stream);
+int sseqs_decode_scan_delims(int64_t n_syms, int64_t n_delims, int32_t* out_pos,
+                             const void* workspace, size_t ws_bytes, cudaStream_t stream);
+
+/* Non-empty segments of n symbols whose '@' sit at delim[0 .. n_delims)
+ * (sseqs/msa.py:237-267; trailing: the symbols after the last '@' form one more):
+ * segment number, length and running sum of length + 1 of each, arrays of
+ * n_delims + 1; info (device, int64[3]): their number, the longest, the residues in all. */
+size_t sseqs_segments_workspace_bytes(int64_t max_segments);
+int sseqs_segments(int64_t n, const int32_t* delim, int64_t n_delims, int trailing,
+                   int32_t* seg_index, int32_t* lengths, int64_t* offsets, int64_t* info,
+                   void* workspace, size_t ws_bytes, cudaStream_t stream);
+
 /* Replaces compress_launcher (sseqs/xbit.cu:73-78, kernel :36-62; wrapper
  * sseqs/xbit_bind.cpp:11-18): out holds (5*n_syms+7)/8 bytes; a partial last
  * group packs missing symbols as 0. */

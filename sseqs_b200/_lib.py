@@ -28,6 +28,11 @@ _SIGNATURES = {
     "sseqs_version": (_I, []),
     "sseqs_max_query_len": (_I, []),
     "sseqs_xbit_decompress": (_I, [_P, _P, _I64, _I64, _P]),
+    "sseqs_decode_scan_workspace_bytes": (_SZ, [_I64]),
+    "sseqs_decode_scan": (_I, [_P, _P, _I64, _I64, _P, _P, _SZ, _P]),
+    "sseqs_decode_scan_delims": (_I, [_I64, _I64, _P, _P, _SZ, _P]),
+    "sseqs_segments_workspace_bytes": (_SZ, [_I64]),
+    "sseqs_segments": (_I, [_I64, _P, _I64, _I, _P, _P, _P, _P, _P, _SZ, _P]),
     "sseqs_xbit_compress": (_I, [_P, _P, _I64, _P]),
     "sseqs_sw_linear": (_I, [_P, _I, _P, _P, _P, _I64, _P, _I, _P]),
     "sseqs_sw_affine": (_I, [_P, _I, _P, _P, _P, _I64, _P, _I, _I, _P]),

@@ -23,7 +23,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from . import select, xbit
+from ._lib import check, lib, ptr, stream_ptr, workspace
 
 CHUNK_BYTES = 1_000_000_000
 
@@ -41,25 +41,6 @@ class Batch:
     maxlen: int
     n_segments: int
     n_residues: int
-
-
-def _effective_length(ascii: torch.Tensor) -> int:
-    """Index after the delimiter that closes the last non-'@' byte."""
-    n = ascii.numel()
-    if n == 0:
-        return 0
-    blk = 1 << 16
-    nb = (n + blk - 1) // blk
-    pad = nb * blk - n
-    a = torch.nn.functional.pad(ascii, (0, pad), value=64) if pad else ascii
-    any_res = (a.view(nb, blk) != 64).any(1)
-    nzb = torch.nonzero(any_res).flatten()
-    if nzb.numel() == 0:
-        return 0
-    b = int(nzb[-1].item())
-    row = a[b * blk:(b + 1) * blk]
-    last = b * blk + int(torch.nonzero(row != 64).flatten()[-1].item())
-    return min(n, last + 2)
 
 
 class Database:
@@ -94,20 +75,42 @@ class Database:
 
     def _add_batch(self, ci, j, ch):
         n_sym = int(self.bs * 8 / 5)
-        full = xbit.decompress(ch, n_sym, j * self.bs)
-        eff = _effective_length(full)
-        if eff == 0:
+        lo = j * self.bs
+        if lo + (5 * n_sym + 7) // 8 > ch.numel():
+            raise ValueError("a batch reaches past its chunk")
+        L, dev, st = lib(), ch.device, stream_ptr()
+        # decode, and note the '@' on the way; one read of (last residue, '@' count)
+        # by the host sizes everything else
+        full = torch.empty(n_sym, dtype=torch.uint8, device=dev)
+        info = torch.empty(5, dtype=torch.int64, device=dev)
+        ws = workspace(L.sseqs_decode_scan_workspace_bytes(n_sym), dev)
+        check(L.sseqs_decode_scan(ptr(ch), ptr(full), n_sym, lo, ptr(info), ptr(ws), ws.numel(),
+                                  st), "decode_scan")
+        last, total = info[:2].tolist()
+        if last < 0:
             return
-        ascii = full[:eff].clone() if eff < full.numel() else full
-        del full
-        delim = select.find_delims(ascii)
-        tab = select.segment_table(ascii, delim)
-        if tab["n_segments"] == 0:
+        # trimmed after the delimiter that closes the last residue; every
+        # symbol past it is '@'
+        eff = min(n_sym, last + 2)
+        nd, trailing = total - (n_sym - eff), int(last + 1 == n_sym)
+        delim = torch.empty(nd, dtype=torch.int32, device=dev)
+        check(L.sseqs_decode_scan_delims(n_sym, nd, ptr(delim), ptr(ws), ws.numel(), st),
+              "decode_scan_delims")
+        seg_index, lengths = (torch.empty(nd + 1, dtype=torch.int32, device=dev)
+                              for _ in range(2))
+        offsets = torch.empty(nd + 1, dtype=torch.int64, device=dev)
+        ws2 = workspace(L.sseqs_segments_workspace_bytes(nd + 1), dev)
+        check(L.sseqs_segments(eff, ptr(delim), nd, trailing, ptr(seg_index), ptr(lengths),
+                               ptr(offsets), ptr(info[2:]), ptr(ws2), ws2.numel(), st), "segments")
+        # a batch that is nearly full keeps its decoded buffer, a mostly empty
+        # one a copy of the part that is used
+        ascii = full[:eff] if 16 * (n_sym - eff) <= n_sym else full[:eff].clone()
+        m, maxlen, res = info[2:].tolist()
+        if m == 0:
             return
-        res = int(tab["lengths"].sum(dtype=torch.int64).item())
         self.n_residues += res
-        self.batches.append(Batch(ci, j, ascii, n_sym, delim, tab["seg_index"], tab["lengths"],
-                                  tab["offsets"], tab["maxlen"], tab["n_segments"], res))
+        self.batches.append(Batch(ci, j, ascii, n_sym, delim, seg_index[:m], lengths[:m],
+                                  offsets[:m], maxlen, m, res))
 
     @classmethod
     def from_file(cls, path: str, chunks: int | None = None, bs: int = CHUNK_BYTES,

@@ -1,0 +1,57 @@
+"""Loading a batch: decode with delimiters noted on the way, and the segment
+table, against numpy restatements (exact)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _symbols(kind, n, rng):
+    a = rng.integers(65, 96, n).astype(np.uint8)
+    if kind == "ends":                 # '@' here and there, first and last symbol a residue
+        a[rng.integers(0, n, max(1, n // 40))] = 64
+        a[0] = a[-1] = 65
+    elif kind == "padded":             # runs of '@', leading and trailing ones
+        a[rng.integers(0, n, max(1, n // 5))] = 64
+        a[:3] = 64
+        a[-(n // 3):] = 64
+    elif kind == "one":                # a single residue
+        a[:] = 64
+        a[n // 2] = 70
+    elif kind == "none":
+        pass
+    elif kind == "blank":
+        a[:] = 64
+    return a
+
+
+@pytest.mark.parametrize("kind", ["ends", "padded", "one", "none", "blank"])
+@pytest.mark.parametrize("bs", [5, 20, 40, 5120, 5125, 10_240, 500_005])
+def test_batches_match_restatement(kind, bs):
+    from sseqs_b200.database import Database
+    rng = np.random.default_rng(bs)
+    n = bs * 8 // 5
+    raw = [_symbols(kind, n, rng) for _ in range(2)]
+    chunk = np.concatenate([O.xbit_compress(a) for a in raw])
+    db = Database([torch.from_numpy(chunk)], bs=bs)
+    want = []
+    for j, a in enumerate(raw):
+        live = np.flatnonzero(a != 64)
+        if live.size:
+            want.append((j, a[:min(n, live[-1] + 2)]))
+    assert [b.index for b in db.batches] == [j for j, _ in want]
+    for b, (j, a) in zip(db.batches, want):
+        seg = O.segment(a)
+        np.testing.assert_array_equal(b.ascii.cpu().numpy(), a)
+        np.testing.assert_array_equal(b.delim.cpu().numpy(), np.flatnonzero(a == 64))
+        np.testing.assert_array_equal(b.lengths.cpu().numpy(), seg["lengths"])
+        np.testing.assert_array_equal(b.offsets.cpu().numpy(), seg["offsets"])
+        d = np.flatnonzero(a == 64)
+        allseg = np.diff(np.concatenate([[-1], d, [a.size] if a[-1] != 64 else []])) - 1
+        np.testing.assert_array_equal(b.seg_index.cpu().numpy(), np.flatnonzero(allseg))
+        assert (b.maxlen, b.n_segments, b.n_residues) == (
+            seg["lengths"].max(), seg["lengths"].size, seg["lengths"].sum())
+    assert db.n_residues == sum(int((a != 64).sum()) for _, a in want)
