@@ -812,6 +812,333 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(2 * TC_BN));
 }
 
+// Epilogue of 16 consecutive columns n .. n + 15 of row m: 32-byte loads and
+// stores (C, C2, aux, res 32-byte aligned, ldc % 16 == 0).
+struct Half16 { uint32_t w[8]; };
+__device__ __forceinline__ Half16 load_half16(const __nv_bfloat16* p) {
+  Half16 r;
+  asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]),
+                 "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ void store_half16(__nv_bfloat16* p, const Half16& r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               :: "l"(p), "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]),
+                  "r"(r.w[5]), "r"(r.w[6]), "r"(r.w[7]) : "memory");
+}
+__device__ __forceinline__ float half_of(const Half16& r, int j) {
+  return __uint_as_float((j & 1) ? (r.w[j >> 1] & 0xffff0000u) : (r.w[j >> 1] << 16));
+}
+template <int EPI>
+__device__ __forceinline__ void epi_store16(const GemmArgs& g, int64_t m, bool keep, int n,
+                                            const float (&acc)[16], const float (&bias)[16],
+                                            const Half16& rs, const Half16& ax) {
+  Half16 c, z;
+#pragma unroll
+  for (int h = 0; h < 8; ++h) {
+    uint32_t cw = 0, zw = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int j = 2 * h + e;
+      float cval = 0.f;
+      __nv_bfloat16 zb = __float2bfloat16_rn(0.f);
+      if (EPI == EPI_BF16) {
+        cval = keep ? acc[j] : 0.f;
+      } else if (EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_GELU_RES) {
+        zb = __float2bfloat16_rn(keep ? acc[j] + bias[j] : 0.f);
+        const float r = (EPI == EPI_BIAS_GELU_RES) ? half_of(rs, j) : 0.f;
+        cval = keep ? gelu_f(__bfloat162float(zb)) + r : 0.f;
+      } else if (EPI == EPI_GELU_GRAD) {
+        cval = keep ? acc[j] * gelu_grad(half_of(ax, j)) : 0.f;
+      } else {   // EPI_GELU_GRAD_RES
+        zb = __float2bfloat16_rn(keep ? acc[j] + half_of(rs, j) : 0.f);
+        cval = keep ? __bfloat162float(zb) * gelu_grad(half_of(ax, j)) : 0.f;
+      }
+      cw |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(cval)) << (16 * e);
+      zw |= (uint32_t)__bfloat16_as_ushort(zb) << (16 * e);
+    }
+    c.w[h] = cw;
+    z.w[h] = zw;
+  }
+  store_half16(static_cast<__nv_bfloat16*>(g.C) + m * g.ldc + n, c);
+  if ((EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_GELU_RES || EPI == EPI_GELU_GRAD_RES) && g.C2)
+    store_half16(g.C2 + m * g.ldc + n, z);
+}
+
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int x, int y4,
+                                            uint32_t mbar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %3, %3, %4}], [%5];"
+      :: "r"(dst), "l"(map), "r"(x), "r"(0), "r"(y4), "r"(mbar) : "memory");
+}
+
+// ------------------------------------------- tcgen05 GEMM of the convolutions
+// The same GEMMs for long overlapping views (row m + 1 starts lda elements after
+// row m, K = taps * lda).  gemm_ws_kernel is bound by its tiles' way from L2 (983
+// KB for a 128 x 256 tile, two thirds of it B).  Here a CTA takes 256 rows and both
+// halves of the columns in turn: the rows are loaded once, as slabs of 64
+// channels x (128 + taps - 1) rows, and tap t reads the slab from its row t on
+// (the swizzle follows the address, so the descriptor just starts t rows, 128
+// bytes each, further); B's half tiles serve both 128-row tiles.  That is 197
+// KB a tile of the same size.  Slab ring (one slot a slab) and B ring are
+// filled in the order of use, slab outermost, so that a slot is refilled while
+// the other slabs' products run; two accumulators of 2 x 128 columns alternate.
+// Barriers, roles and bounded waits as in gemm_ws_kernel.
+//
+// The epilogue reads 16 rows x 64 columns at a time in the layout in which
+// lane l holds columns 8i + 2(l % 4) + e of rows l / 4 and l / 4 + 8.  B's rows are
+// brought in in the order that makes these 16 consecutive output columns (a 5D
+// tensor map: 2, 4 and 8 rows at strides 1, 16 and 2), so a lane's loads and
+// stores are whole 32-byte sectors and 4 lanes' a line; a row to a lane, as in
+// gemm_ws_kernel, touched 32 lines an instruction and kept the load-store unit
+// busier than the products the tensor pipe.
+//
+// Measured (5.9M rows, K = 1280): GELU + residual 4.48 -> 3.67 ms a layer (868 ->
+// 1060 TFLOP/s; the power-capped cuBLAS rate is 1353), of which the slabs gave
+// 0.65 and the epilogue 0.16 (in a training step, which writes Z too, 0.37 -> 0.31
+// ms a layer for the epilogue alone).  What bounds it now: M = 128, N = 128 products read
+// 128 bytes of shared memory a clock, all it has, at the clock the power cap leaves.
+constexpr int CV_SLABS = 4, CV_SLAB_ROWS = 136, CV_MAX_TAPS = CV_SLAB_ROWS - 127;
+constexpr int CV_A_BYTES = CV_SLAB_ROWS * 128;             // one tile's slab
+constexpr int CV_B_STAGES = 5, CV_B_BYTES = 128 * TC_BK * 2;
+constexpr size_t CV_SMEM =
+    (size_t)CV_SLABS * 2 * CV_A_BYTES + (size_t)CV_B_STAGES * CV_B_BYTES + 1024;
+// as kIdescBf16 with N = 128
+constexpr uint32_t kIdescCv = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) |
+                              ((128u >> 4) << 24);
+
+template <int EPI>
+__global__ void __launch_bounds__(WS_THREADS, 1)
+    gemm_conv_kernel(const __grid_constant__ CUtensorMap map_a,
+                     const __grid_constant__ CUtensorMap map_b, GemmArgs g, int slabs, int taps,
+                     int* err) {
+  extern __shared__ __align__(1024) unsigned char cvm[];
+  const uint32_t raw = smem_u32(cvm);
+  unsigned char* sa = cvm + ((1024 - (raw & 1023)) & 1023);
+  unsigned char* sb = sa + CV_SLABS * 2 * CV_A_BYTES;
+  __shared__ __align__(8) uint64_t a_full[CV_SLABS], a_empty[CV_SLABS];
+  __shared__ __align__(8) uint64_t b_full[CV_B_STAGES], b_empty[CV_B_STAGES];
+  __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], mma_done;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int abort_s;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t npairs = (g.M + 255) / 256;
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&tmem_base_s)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (tid == 0) {
+    auto init = [](uint64_t* b, int count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(b)), "r"(count));
+    };
+    for (int s = 0; s < CV_SLABS; ++s) { init(&a_full[s], 1); init(&a_empty[s], 1); }
+    for (int s = 0; s < CV_B_STAGES; ++s) { init(&b_full[s], 1); init(&b_empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { init(&acc_full[b], 1); init(&acc_empty[b], WS_EPI_WARPS); }
+    init(&mma_done, 1);
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  auto fail = [&]() {
+    abort_s = 1;
+    atomicExch(err, 1);
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ loader
+    if (lane == 0) {
+      asm volatile("prefetch.tensormap [%0];" :: "l"(&map_a) : "memory");
+      asm volatile("prefetch.tensormap [%0];" :: "l"(&map_b) : "memory");
+      const uint32_t a_bytes = 2u * 128u * (uint32_t)(127 + taps);
+      uint32_t a_loads[CV_SLABS] = {}, b_loads = 0;   // slabs by slot, B tiles so far
+      bool ok = true;
+      for (int64_t p = blockIdx.x; p < npairs && ok; p += gridDim.x) {
+        for (int hs = 0; hs < 2 * slabs && ok; ++hs) {
+          const int h = hs >= slabs, s = h ? hs - slabs : hs;
+          if (h == 0) {
+            ok = mbar_wait(smem_u32(&a_empty[s]), (a_loads[s] & 1u) ^ 1u);
+            if (!ok) { fail(); break; }
+            const uint32_t fb = smem_u32(&a_full[s]);
+            mbar_expect_tx(fb, a_bytes);
+            const uint32_t dst = smem_u32(sa + s * 2 * CV_A_BYTES);
+            tma_load_2d(dst, &map_a, s * 64, (int)(p * 256), fb);
+            tma_load_2d(dst + CV_A_BYTES, &map_a, s * 64, (int)(p * 256 + 128), fb);
+            ++a_loads[s];
+          }
+          for (int t = 0; t < taps; ++t) {
+            const uint32_t stage = b_loads % CV_B_STAGES;
+            ok = mbar_wait(smem_u32(&b_empty[stage]), ((b_loads / CV_B_STAGES) & 1u) ^ 1u);
+            if (!ok) { fail(); break; }
+            const uint32_t fb = smem_u32(&b_full[stage]);
+            mbar_expect_tx(fb, (uint32_t)CV_B_BYTES);
+            tma_load_5d(smem_u32(sb + stage * CV_B_BYTES), &map_b, (t * slabs + s) * 64, h * 2, fb);
+            ++b_loads;
+          }
+          if (abort_s) ok = false;
+        }
+      }
+      // before exit every issued load has landed (see gemm_ws_kernel)
+      if (abort_s) {
+        for (uint32_t s = 0; s < CV_B_STAGES; ++s) {
+          const uint32_t n = (b_loads + CV_B_STAGES - 1 - s) / CV_B_STAGES;
+          if (n > 0) mbar_wait(smem_u32(&b_full[s]), (n - 1) & 1u);
+        }
+        for (int s = 0; s < slabs; ++s)
+          if (a_loads[s] > 0) mbar_wait(smem_u32(&a_full[s]), (a_loads[s] - 1) & 1u);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issue
+    if (lane == 0) {
+      uint32_t pairs = 0, tiles = 0, units = 0;
+      bool any = false, ok = true;
+      for (int64_t p = blockIdx.x; p < npairs && ok; p += gridDim.x, ++pairs) {
+        for (int h = 0; h < 2 && ok; ++h, ++units) {
+          const uint32_t b = units & 1u;
+          if (!mbar_wait(smem_u32(&acc_empty[b]), ((units >> 1) & 1u) ^ 1u)) { fail(); ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          for (int s = 0; s < slabs && ok; ++s) {
+            if (h == 0 && !mbar_wait(smem_u32(&a_full[s]), pairs & 1u)) { fail(); ok = false; break; }
+            const uint32_t a0 = smem_u32(sa + s * 2 * CV_A_BYTES);
+            for (int t = 0; t < taps; ++t, ++tiles) {
+              const uint32_t stage = tiles % CV_B_STAGES;
+              if (!mbar_wait(smem_u32(&b_full[stage]), (tiles / CV_B_STAGES) & 1u)) {
+                fail();
+                ok = false;
+                break;
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t b0 = smem_u32(sb + stage * CV_B_BYTES);
+#pragma unroll
+              for (int ks = 0; ks < TC_BK / 16; ++ks) {
+                const uint64_t db = umma_desc_sw128(b0 + ks * 32);
+                const uint32_t accum = (s > 0 || t > 0 || ks > 0) ? 1u : 0u;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const uint64_t da = umma_desc_sw128(a0 + i * CV_A_BYTES + t * 128 + ks * 32);
+                  asm volatile(
+                      "{\n\t.reg .pred p;\n\t"
+                      "setp.ne.b32 p, %4, 0;\n\t"
+                      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                      :: "r"(tmem + b * 256u + (uint32_t)(i * 128)), "l"(da), "l"(db),
+                         "r"(kIdescCv), "r"(accum));
+                }
+              }
+              any = true;
+              commit_to(smem_u32(&b_empty[stage]), 1u);
+            }
+            if (ok && h == 1) commit_to(smem_u32(&a_empty[s]), 1u);
+          }
+          if (!ok || abort_s) { ok = false; break; }
+          commit_to(smem_u32(&acc_full[b]), 1u);
+        }
+      }
+      // every MMA issued is complete before the tensor memory is freed
+      if (any) {
+        commit_to(smem_u32(&mma_done), 1u);
+        if (!mbar_wait(smem_u32(&mma_done), 0)) fail();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue
+    const int e = warp - 2, q = warp & 3, i = e >> 2;   // tile i of the pair, rows 32q ..
+    const int sub = lane & 3;                           // columns 16 sub .. of every 64
+    uint32_t units = 0;
+    bool ok = true;
+    for (int64_t p = blockIdx.x; p < npairs && ok; p += gridDim.x) {
+      // this lane's rows m0 + 8k, k < 4
+      const int64_t m0 = p * 256 + i * 128 + q * 32 + (lane >> 2);
+      bool keep[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t m = m0 + 8 * k;
+        keep[k] = m < g.M && (g.row_mask ? g.row_mask[m] != 0 : true);
+      }
+      for (int h = 0; h < 2; ++h, ++units) {
+        const uint32_t b = units & 1u;
+        // residual and pre-activation rows of the first step are read before the
+        // wait, those of the next one before each step's arithmetic
+        Half16 rs[2] = {}, ax[2] = {};
+        auto fetch = [&](int step) {
+          const int n = h * 128 + (step >> 1) * 64 + 16 * sub;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int64_t m = m0 + 16 * (step & 1) + 8 * k;
+            if (m < g.M) {
+              if (EPI == EPI_BIAS_GELU_RES || EPI == EPI_GELU_GRAD_RES)
+                rs[k] = load_half16(g.res + m * g.ldc + n);
+              if (EPI == EPI_GELU_GRAD || EPI == EPI_GELU_GRAD_RES)
+                ax[k] = load_half16(g.aux + m * g.ldc + n);
+            }
+          }
+        };
+        fetch(0);
+        if (!mbar_wait(smem_u32(&acc_full[b]), (units >> 1) & 1u)) {
+          if (lane == 0) fail();
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+        for (int step = 0; step < 4; ++step) {          // (64-column block, 16-row half)
+          const int blk = step >> 1, half = step & 1;
+          uint32_t v[32];
+          const uint32_t taddr = tmem + ((uint32_t)(q * 32 + half * 16) << 16) + b * 256u +
+                                 (uint32_t)(i * 128 + blk * 64);
+          asm volatile(
+              "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+              "%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+                "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+                "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+                "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+                "=r"(v[31])
+              : "r"(taddr));
+          const int n = h * 128 + blk * 64 + 16 * sub;
+          float bias[16] = {};
+          if (EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_GELU_RES) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float4 x = __ldg(reinterpret_cast<const float4*>(g.bias + n) + j);
+              bias[4 * j] = x.x; bias[4 * j + 1] = x.y; bias[4 * j + 2] = x.z; bias[4 * j + 3] = x.w;
+            }
+          }
+          const Half16 r0 = rs[0], r1 = rs[1], a0 = ax[0], a1 = ax[1];
+          if (step < 3) fetch(step + 1);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          float lo[16], hi[16];                         // rows +0 and +8
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            lo[2 * j] = __uint_as_float(v[4 * j]);
+            lo[2 * j + 1] = __uint_as_float(v[4 * j + 1]);
+            hi[2 * j] = __uint_as_float(v[4 * j + 2]);
+            hi[2 * j + 1] = __uint_as_float(v[4 * j + 3]);
+          }
+          const int64_t m = m0 + 16 * half;
+          if (m < g.M) epi_store16<EPI>(g, m, half ? keep[2] : keep[0], n, lo, bias, r0, a0);
+          if (m + 8 < g.M) epi_store16<EPI>(g, m + 8, half ? keep[3] : keep[1], n, hi, bias, r1, a1);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+        if (abort_s) { ok = false; break; }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512));
+}
+
 // ------------------------------------------------- tcgen05 weight gradient
 // C[M x 256] += A^T B with A [K][M] and B [K][256] (bf16, K = positions, the
 // weight gradients of the 256-channel layers): both operands are MN-major, as
@@ -1972,6 +2299,61 @@ int launch_tc_ws(const GemmArgs& g, cudaStream_t stream) {
   return status_of(cudaGetLastError());
 }
 
+// Tensor map of a 256-row bf16 operand for gemm_conv_kernel: boxes of 64 columns x
+// 128 rows, the rows of every 64 in the order 16q + 2i + e for (i, q, e), e
+// fastest (i < 8, q < 4, e < 2).
+static bool make_map_cols(CUtensorMap* map, const void* base, int64_t K, int64_t ld) {
+  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  if (!encode) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) !=
+            cudaSuccess || q != cudaDriverEntryPointSuccess || !fn)
+      return false;
+    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }
+  const cuuint64_t row = (cuuint64_t)ld * 2;
+  const cuuint64_t dims[5] = {(cuuint64_t)K, 2, 4, 8, 4};
+  const cuuint64_t strides[4] = {row, 16 * row, 2 * row, 64 * row};
+  const cuuint32_t box[5] = {64, 2, 4, 8, 2};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides,
+                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
+}
+
+// The slab kernel applies to overlapping views of whole 64-channel slabs (at most
+// CV_SLABS) and CV_MAX_TAPS taps, with two pairs of 128-row tiles to an SM
+// or more: a pair takes twice a tile's time, so that below that the single tiles of
+// gemm_ws_kernel fill the SMs better; and to 32-byte aligned rows.
+static bool conv_applies(const GemmArgs& g) {
+  auto al = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
+  if (!al(g.C, 32) || !al(g.C2, 32) || !al(g.aux, 32) || !al(g.res, 32) || g.ldc % 16 != 0 ||
+      !al(g.bias, 16))
+    return false;
+  return g.lda < g.K && g.lda % 64 == 0 && g.lda / 64 <= CV_SLABS && g.K % g.lda == 0 &&
+         g.K / g.lda <= CV_MAX_TAPS && g.M >= (int64_t)512 * device_sm_count();
+}
+
+template <int EPI>
+int launch_conv(const GemmArgs& g, cudaStream_t stream) {
+  int* err = tc_error_flag();
+  if (!err) return SSEQS_ERR_CUDA;
+  const int slabs = (int)(g.lda / 64), taps = (int)(g.K / g.lda);
+  CUtensorMap ma, mb;
+  if (!make_map(&ma, g.A, g.lda, g.M + taps - 1, g.lda, 127 + taps) ||
+      !make_map_cols(&mb, g.B, g.K, g.ldb))
+    return SSEQS_ERR_CUDA;
+  auto fn = gemm_conv_kernel<EPI>;
+  if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)CV_SMEM) != cudaSuccess)
+    return SSEQS_ERR_CUDA;
+  const int grid = (int)std::min<int64_t>((g.M + 255) / 256, device_sm_count());
+  { fn<<<grid, WS_THREADS, CV_SMEM, stream>>>(ma, mb, g, slabs, taps, err); count_launches(1); }
+  return status_of(cudaGetLastError());
+}
+
 // The MN-major kernel applies when 64-column boxes of A stay inside its rows
 // (a plain matrix, or an overlapping view with lda % 64 == 0) and C takes
 // 16-byte reductions.
@@ -2057,6 +2439,15 @@ extern "C" int sseqs_gemm_bf16(int a_t, int b_t, int epilogue, int64_t M, int64_
       (!res || (reinterpret_cast<uintptr_t>(res) & 15) == 0) &&
       (!aux || (reinterpret_cast<uintptr_t>(aux) & 15) == 0) &&
       epilogue != EPI_F32 && epilogue != EPI_F32_ADD) {
+    if (ws_applies(g) && conv_applies(g)) {
+      switch (epilogue) {
+        case EPI_BF16: return launch_conv<EPI_BF16>(g, stream);
+        case EPI_BIAS_GELU: return launch_conv<EPI_BIAS_GELU>(g, stream);
+        case EPI_GELU_GRAD: return launch_conv<EPI_GELU_GRAD>(g, stream);
+        case EPI_BIAS_GELU_RES: return launch_conv<EPI_BIAS_GELU_RES>(g, stream);
+        case EPI_GELU_GRAD_RES: return launch_conv<EPI_GELU_GRAD_RES>(g, stream);
+      }
+    }
     if (ws_applies(g)) {
       switch (epilogue) {
         case EPI_BF16: return launch_tc_ws<EPI_BF16>(g, stream);

@@ -1,0 +1,52 @@
+"""The slab-fed tcgen05 GEMM of long overlapping views, at its edges.
+
+fp32 sums of exact bf16 products (K / 16 tensor-core additions, each within
+2^-22 of the magnitudes summed), rounded to bf16 (2^-8 of the value)."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+FIRST = 512 * 148          # rows from which the slab kernel is taken on 148 SMs
+
+
+@pytest.mark.parametrize("M", [FIRST, FIRST + 1, FIRST + 129, FIRST + 255, 3 * FIRST + 300])
+@pytest.mark.parametrize("lda,taps", [(256, 5), (64, 2), (128, 9), (192, 3)])
+def test_slab_gemm_matches_64_bit_rows(M, lda, taps):
+    from sseqs_b200 import _lib, learned
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + lda + taps)
+    K, N = lda * taps, 256
+    X = torch.randn(M + taps - 1, lda, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    res = torch.randn(M, N, generator=g, device="cuda").to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    mask = (torch.rand(M, generator=g, device="cuda") > 0.2).to(torch.uint8)
+    plain = torch.full((M + 1, N), 3, dtype=torch.bfloat16, device="cuda")
+    fused, Z = (torch.zeros(M, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    learned._gemm(0, 0, learned._EPI_BF16, M, N, K, X.data_ptr(), lda, B.data_ptr(), K,
+                  plain.data_ptr(), N)
+    learned._gemm(0, 0, learned._EPI_BIAS_GELU_RES, M, N, K, X.data_ptr(), lda, B.data_ptr(), K,
+                  fused.data_ptr(), N, Z.data_ptr(), bias, None, mask, res.data_ptr())
+    torch.cuda.synchronize()
+    flag = ctypes.c_int(-1)
+    _lib.check(_lib.lib().sseqs_gemm_error(ctypes.byref(flag)))
+    assert flag.value == 0
+    assert (plain[M] == 3).all()                       # nothing past the last row
+    # rows of the first, some middle and the last tiles
+    rows = torch.cat([torch.arange(0, 700), torch.arange(M // 2, M // 2 + 700),
+                      torch.arange(M - 700, M)]).cuda()
+    A = torch.as_strided(X, (M, K), (lda, 1))[rows].double()
+    exp = A @ B.double().T
+    size = A.abs() @ B.double().abs().T
+    tol = 2.0 ** -8 * exp.abs() + K / 16 * 2.0 ** -22 * size
+    assert ((plain[rows].double() - exp).abs() <= tol).all()
+    z = torch.where(mask[rows].bool()[:, None], exp + bias.double(), 0.0)
+    assert ((Z[rows].double() - z).abs() <= tol + 2.0 ** -8 * (z.abs() + 1e-30)).all()
+    zb = Z[rows].float()
+    y = torch.nn.functional.gelu(zb, approximate="tanh") + res[rows].float()
+    y = torch.where(mask[rows].bool()[:, None], y, 0.0)
+    # tanh.approx is within 2^-10.9 of tanh; the sum is rounded to bf16
+    assert ((fused[rows].float() - y).abs() <= 2.0 ** -8 * y.abs() + 2.0 ** -11 * zb.abs() +
+            1e-6).all()
