@@ -168,6 +168,32 @@ int sseqs_sw_scan_queries(int affine, int n_queries, int tpt, const uint8_t* que
                           uint32_t* tickets, cudaStream_t stream);
 
 /* ------------------------------------------------------------ selection */
+/* The three scans above with the order in which targets are taken: a
+ * permutation of 0 .. n_targets - 1 (device, int32; null: as they stand; used
+ * for up to 2^30 targets).  Scores and their places do not depend on it;
+ * taking the longest targets first is faster.  sseqs_length_order writes such an order for
+ * targets good_idx[t] (null: g0 + t): by window length, in steps of 8 residues,
+ * longest first (all of 2040 or more alike), no order inside a step. */
+int sseqs_sw_scan_ordered(int affine, const uint8_t* query_idx, int query_len,
+                          const int32_t* good_idx, int32_t g0, int64_t n_targets,
+                          const int32_t* order, const uint8_t* ascii, const int32_t* delim,
+                          int skip, int32_t* out, int gap_a, int gap_b, cudaStream_t stream);
+int sseqs_sw_scan_both_ordered(const uint8_t* query_idx, int query_len, const int32_t* good_idx,
+                               int32_t g0, int64_t n_targets, const int32_t* order,
+                               const uint8_t* ascii, const int32_t* delim, int affine_skip,
+                               int32_t* out_linear, int32_t* out_affine, int gap, int gap_open,
+                               int gap_extend, cudaStream_t stream);
+int sseqs_sw_scan_queries_ordered(int affine, int n_queries, int tpt, const uint8_t* queries,
+                                  int64_t query_stride, const int32_t* query_lens,
+                                  const int32_t* good_idx, int64_t idx_stride, int32_t g0,
+                                  int64_t n_targets, const int32_t* order, const uint8_t* ascii,
+                                  const int32_t* delim, int skip, int32_t* out,
+                                  int64_t out_stride, int gap_a, int gap_b, uint32_t* tickets,
+                                  cudaStream_t stream);
+size_t sseqs_length_order_workspace_bytes(void);
+int sseqs_length_order(const int32_t* delim, const int32_t* good_idx, int32_t g0, int64_t n,
+                       int32_t* order, void* workspace, size_t ws_bytes, cudaStream_t stream);
+
 /* Positions (int32, increasing) of every '@' (64) byte of a decoded batch:
  * replaces `delim_pos = arange[ascii == 64]` (sseqs/msa.py:227).  Writes at
  * most max_out positions and the total count to *count (device int64).

@@ -41,6 +41,14 @@ _SIGNATURES = {
                                 _P]),
     "sseqs_sw_scan_queries": (_I, [_I, _I, _I, _P, _I64, _P, _P, _I64, ctypes.c_int32, _I64,
                                    _P, _P, _I, _P, _I64, _I, _I, _P, _P]),
+    "sseqs_sw_scan_ordered": (_I, [_I, _P, _I, _P, ctypes.c_int32, _I64, _P, _P, _P, _I, _P, _I,
+                                   _I, _P]),
+    "sseqs_sw_scan_both_ordered": (_I, [_P, _I, _P, ctypes.c_int32, _I64, _P, _P, _P, _I, _P, _P,
+                                        _I, _I, _I, _P]),
+    "sseqs_sw_scan_queries_ordered": (_I, [_I, _I, _I, _P, _I64, _P, _P, _I64, ctypes.c_int32,
+                                           _I64, _P, _P, _P, _I, _P, _I64, _I, _I, _P, _P]),
+    "sseqs_length_order_workspace_bytes": (_SZ, []),
+    "sseqs_length_order": (_I, [_P, _P, ctypes.c_int32, _I64, _P, _P, _SZ, _P]),
     "sseqs_find_delims_workspace_bytes": (_SZ, [_I64]),
     "sseqs_find_delims": (_I, [_P, _I64, _P, _I64, _P, _P, _SZ, _P]),
     "sseqs_segment_table_workspace_bytes": (_SZ, [_I64]),

@@ -36,14 +36,16 @@ def sw_scan_queries(queries: torch.Tensor, lens: torch.Tensor, tpt: int, ascii: 
                     delim: torch.Tensor, *, affine: bool, good_idx: torch.Tensor | None = None,
                     g0: int = 0, n_targets: int | None = None, skip: int = 0, gap_a: int = -1,
                     gap_b: int = 0, out: torch.Tensor | None = None,
-                    tickets: torch.Tensor | None = None) -> torch.Tensor:
+                    tickets: torch.Tensor | None = None,
+                    order: torch.Tensor | None = None) -> torch.Tensor:
     """Scores ``[len(lens), n]`` of several queries of stripe width ``tpt``.
 
     ``queries`` is a uint8 device tensor ``[>= len(lens), stride]`` of residue
     classes, row i holding ``lens[i]`` of them (``lens``: device int32, every
     ``ceil(len/32) == tpt``; a row that breaks this is filled with INT32_MIN);
     target selection and gap parameters are those of ``sw.sw_scan``, except
-    that a 2-D ``good_idx`` gives every query its own row of targets.
+    that a 2-D ``good_idx`` gives every query its own row of targets (``order``
+    is one for all of them).
     """
     nq = lens.numel()
     idx_stride = 0
@@ -60,11 +62,12 @@ def sw_scan_queries(queries: torch.Tensor, lens: torch.Tensor, tpt: int, ascii: 
         out = torch.empty((nq, max(n, 1)), dtype=torch.int32, device=ascii.device)
     if tickets is None:
         tickets = torch.empty(max(nq, 1), dtype=torch.int32, device=ascii.device)
-    check(lib().sseqs_sw_scan_queries(1 if affine else 0, nq, int(tpt), ptr(queries),
-                                      queries.stride(0), ptr(lens), ptr(good_idx), idx_stride,
-                                      int(g0), n,
-                                      ptr(ascii), ptr(delim), int(skip), ptr(out), out.stride(0),
-                                      int(gap_a), int(gap_b), ptr(tickets), stream_ptr()),
+    check(lib().sseqs_sw_scan_queries_ordered(1 if affine else 0, nq, int(tpt), ptr(queries),
+                                              queries.stride(0), ptr(lens), ptr(good_idx),
+                                              idx_stride, int(g0), n, _sw._order(order, n),
+                                              ptr(ascii), ptr(delim), int(skip), ptr(out),
+                                              out.stride(0), int(gap_a), int(gap_b),
+                                              ptr(tickets), stream_ptr()),
           "sw_scan_queries")
     return out
 
@@ -129,7 +132,7 @@ class _GroupPlan:
                 continue
             sw_scan_queries(self.q, self.lens, self.tpt, batch.ascii, batch.delim, affine=True,
                             g0=1, n_targets=n, skip=1, gap_a=open_, gap_b=ext,
-                            out=self.scores, tickets=self.tickets)
+                            out=self.scores, tickets=self.tickets, order=batch.order)
             for i in range(self.nq):
                 row = self.scores[i, :n]
                 select.topk_indices(row, k, out=self.idx[bi][i], ws=self.ws)

@@ -881,8 +881,8 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 // halves of the columns in turn: the rows are loaded once, as slabs of 64
 // channels x (128 + taps - 1) rows, and tap t reads the slab from its row t on
 // (the swizzle follows the address, so the descriptor just starts t rows, 128
-// bytes each, further); B's half tiles serve both 128-row tiles.  That is 197
-// KB a tile of the same size.  Slab ring (one slot a slab) and B ring are
+// bytes each, further); B's half tiles serve both 128-row tiles.  That is 395
+// KB for as many products.  Slab ring (one slot a slab) and B ring are
 // filled in the order of use, slab outermost, so that a slot is refilled while
 // the other slabs' products run; two accumulators of 2 x 128 columns alternate.
 // Barriers, roles and bounded waits as in gemm_ws_kernel.

@@ -638,6 +638,91 @@ extern "C" int sseqs_gather_windows(const uint8_t* ascii, const int64_t* offsets
   return status_of(cudaGetLastError());
 }
 
+// ------------------------------------------------------- order by length
+// Counting sort of targets by window length: bins of 8 residues, the longest
+// first.  The last block of the count turns the bins into offsets; a block of
+// the second launch reserves its share of a bin with one atomic.
+namespace sseqs {
+namespace {
+constexpr int kLenBins = 256, kLenItems = 8, kLenTile = kSelThreads * kLenItems;
+struct LenCtl {
+  uint32_t done;
+  uint32_t bin[kLenBins];
+};
+__device__ __forceinline__ int length_bin(const int32_t* delim, const int32_t* idx, int32_t g0,
+                                          int64_t t) {
+  const int32_t g = idx ? idx[t] : (int32_t)(g0 + t);
+  const int64_t len = (int64_t)delim[g] - (g == 0 ? -1 : (int64_t)delim[g - 1]) - 1;
+  return kLenBins - 1 - (int)min((int64_t)(kLenBins - 1), max((int64_t)0, len) >> 3);
+}
+__global__ void __launch_bounds__(kSelThreads)
+    length_count_kernel(const int32_t* delim, const int32_t* idx, int32_t g0, int64_t n,
+                        LenCtl* ctl) {
+  __shared__ uint32_t h[kLenBins];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  for (int64_t t = (int64_t)blockIdx.x * kSelThreads + threadIdx.x; t < n;
+       t += (int64_t)gridDim.x * kSelThreads)
+    atomicAdd(&h[length_bin(delim, idx, g0, t)], 1u);
+  __syncthreads();
+  if (h[threadIdx.x]) atomicAdd(&ctl->bin[threadIdx.x], h[threadIdx.x]);
+  if (!last_block(&ctl->done)) return;
+  int64_t ex;
+  block_exclusive_scan((int64_t)__ldcg(&ctl->bin[threadIdx.x]), &ex);
+  ctl->bin[threadIdx.x] = (uint32_t)ex;
+}
+__global__ void __launch_bounds__(kSelThreads)
+    length_scatter_kernel(const int32_t* delim, const int32_t* idx, int32_t g0, int64_t n,
+                          LenCtl* ctl, int32_t* order) {
+  __shared__ uint32_t h[kLenBins];
+  for (int64_t b = (int64_t)blockIdx.x * kLenTile; b < n; b += (int64_t)gridDim.x * kLenTile) {
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    int bin[kLenItems];
+    uint32_t rank[kLenItems];
+#pragma unroll
+    for (int i = 0; i < kLenItems; ++i) {
+      const int64_t t = b + i * kSelThreads + threadIdx.x;
+      bin[i] = t < n ? length_bin(delim, idx, g0, t) : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < kLenItems; ++i) rank[i] = bin[i] >= 0 ? atomicAdd(&h[bin[i]], 1u) : 0u;
+    __syncthreads();
+    const uint32_t mine = h[threadIdx.x];
+    const uint32_t base = mine ? atomicAdd(&ctl->bin[threadIdx.x], mine) : 0u;
+    __syncthreads();
+    h[threadIdx.x] = base;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kLenItems; ++i)
+      if (bin[i] >= 0)
+        order[h[bin[i]] + rank[i]] = (int32_t)(b + i * kSelThreads + threadIdx.x);
+    __syncthreads();
+  }
+}
+}  // namespace
+}  // namespace sseqs
+
+extern "C" size_t sseqs_length_order_workspace_bytes(void) { return align256(sizeof(LenCtl)); }
+
+extern "C" int sseqs_length_order(const int32_t* delim, const int32_t* good_idx, int32_t g0,
+                                  int64_t n, int32_t* order, void* workspace, size_t ws_bytes,
+                                  cudaStream_t stream) {
+  if (n < 0 || g0 < 0) return SSEQS_ERR_ARG;
+  if (n == 0) return SSEQS_OK;
+  if (!delim || !order) return SSEQS_ERR_ARG;
+  if (n > INT32_MAX) return SSEQS_ERR_UNSUPPORTED;
+  if (!workspace || ws_bytes < sseqs_length_order_workspace_bytes()) return SSEQS_ERR_WORKSPACE;
+  LenCtl* ctl = static_cast<LenCtl*>(workspace);
+  if (cudaMemsetAsync(ctl, 0, sizeof(LenCtl), stream) != cudaSuccess) return SSEQS_ERR_CUDA;
+  const int grid = (int)std::min<int64_t>((n + kLenTile - 1) / kLenTile,
+                                          (int64_t)device_sm_count() * 8);
+  { length_count_kernel<<<grid, kSelThreads, 0, stream>>>(delim, good_idx, g0, n, ctl); count_launches(1); }
+  { length_scatter_kernel<<<grid, kSelThreads, 0, stream>>>(delim, good_idx, g0, n, ctl, order);
+    count_launches(1); }
+  return status_of(cudaGetLastError());
+}
+
 // ------------------------------------------------------ segment packing
 // Segment i (bytes [src[i], src[i] + len[i]) of the buffer bases[part[i]])
 // goes to out[dst[i] ..], followed by one '@'.  One warp per segment: the

@@ -172,6 +172,7 @@ int launch_stream(SwArgs a, int mode, const QueryTable* qt, cudaStream_t stream)
     if (a.out2) p.out2 = a.out2 + t0;
     if (a.idx) p.idx = a.idx + t0;
     else p.g0 = (int32_t)(a.g0 + t0);
+    if (a.n > kPiece) p.order = nullptr;      // a piece is not a permutation of its own
     p.ticket = qt ? tickets : ticket_slot(dev);
     if (!p.ticket) return SSEQS_ERR_CUDA;
     if (cudaMemsetAsync(p.ticket, 0, sizeof(unsigned int) * ny, stream) != cudaSuccess)
@@ -304,20 +305,31 @@ extern "C" int sseqs_sw_affine(const uint8_t* query_idx, int query_len, const in
   return run(true, a, stream);
 }
 
+extern "C" int sseqs_sw_scan_ordered(int affine, const uint8_t* query_idx, int query_len,
+                                     const int32_t* good_idx, int32_t g0, int64_t n_targets,
+                                     const int32_t* order, const uint8_t* ascii,
+                                     const int32_t* delim, int skip, int32_t* out, int gap_a,
+                                     int gap_b, cudaStream_t stream) {
+  if (skip < 0 || g0 < 0) return SSEQS_ERR_ARG;
+  SwArgs a{query_idx, query_len, good_idx, g0, n_targets, ascii, delim, skip, out, gap_a, gap_b};
+  a.order = order;
+  return run(affine != 0, a, stream);
+}
+
 extern "C" int sseqs_sw_scan(int affine, const uint8_t* query_idx, int query_len,
                              const int32_t* good_idx, int32_t g0, int64_t n_targets,
                              const uint8_t* ascii, const int32_t* delim, int skip, int32_t* out,
                              int gap_a, int gap_b, cudaStream_t stream) {
-  if (skip < 0 || g0 < 0) return SSEQS_ERR_ARG;
-  SwArgs a{query_idx, query_len, good_idx, g0, n_targets, ascii, delim, skip, out, gap_a, gap_b};
-  return run(affine != 0, a, stream);
+  return sseqs_sw_scan_ordered(affine, query_idx, query_len, good_idx, g0, n_targets, nullptr,
+                               ascii, delim, skip, out, gap_a, gap_b, stream);
 }
 
-extern "C" int sseqs_sw_scan_both(const uint8_t* query_idx, int query_len,
-                                  const int32_t* good_idx, int32_t g0, int64_t n_targets,
-                                  const uint8_t* ascii, const int32_t* delim, int affine_skip,
-                                  int32_t* out_linear, int32_t* out_affine, int gap,
-                                  int gap_open, int gap_extend, cudaStream_t stream) {
+extern "C" int sseqs_sw_scan_both_ordered(const uint8_t* query_idx, int query_len,
+                                          const int32_t* good_idx, int32_t g0, int64_t n_targets,
+                                          const int32_t* order, const uint8_t* ascii,
+                                          const int32_t* delim, int affine_skip,
+                                          int32_t* out_linear, int32_t* out_affine, int gap,
+                                          int gap_open, int gap_extend, cudaStream_t stream) {
   if (g0 < 0 || n_targets < 0 || (affine_skip != 0 && affine_skip != 1)) return SSEQS_ERR_ARG;
   if (n_targets == 0) return SSEQS_OK;
   if (!out_linear || !out_affine || !delim || !ascii) return SSEQS_ERR_ARG;
@@ -334,6 +346,7 @@ extern "C" int sseqs_sw_scan_both(const uint8_t* query_idx, int query_len,
     return SSEQS_ERR_UNSUPPORTED;
   SwArgs a{query_idx, query_len, good_idx, g0, n_targets, ascii, delim, 0, out_linear, gap,
            gap_open};
+  a.order = order;
   if ((query_len + 31) / 32 > kMaxFusedTpt) {   // no fused kernel: the two scans in turn
     const int st = launch_stream(a, kLin, nullptr, stream);
     if (st != SSEQS_OK) return st;
@@ -350,10 +363,21 @@ extern "C" int sseqs_sw_scan_both(const uint8_t* query_idx, int query_len,
   return launch_stream(a, kBoth, nullptr, stream);
 }
 
-extern "C" int sseqs_sw_scan_queries(int affine, int n_queries, int tpt, const uint8_t* queries,
+extern "C" int sseqs_sw_scan_both(const uint8_t* query_idx, int query_len,
+                                  const int32_t* good_idx, int32_t g0, int64_t n_targets,
+                                  const uint8_t* ascii, const int32_t* delim, int affine_skip,
+                                  int32_t* out_linear, int32_t* out_affine, int gap,
+                                  int gap_open, int gap_extend, cudaStream_t stream) {
+  return sseqs_sw_scan_both_ordered(query_idx, query_len, good_idx, g0, n_targets, nullptr, ascii,
+                                    delim, affine_skip, out_linear, out_affine, gap, gap_open,
+                                    gap_extend, stream);
+}
+
+extern "C" int sseqs_sw_scan_queries_ordered(int affine, int n_queries, int tpt,
+                                     const uint8_t* queries,
                                      int64_t query_stride, const int32_t* query_lens,
                                      const int32_t* good_idx, int64_t idx_stride, int32_t g0,
-                                     int64_t n_targets,
+                                     int64_t n_targets, const int32_t* order,
                                      const uint8_t* ascii, const int32_t* delim, int skip,
                                      int32_t* out, int64_t out_stride, int gap_a, int gap_b,
                                      uint32_t* tickets, cudaStream_t stream) {
@@ -388,6 +412,7 @@ extern "C" int sseqs_sw_scan_queries(int affine, int n_queries, int tpt, const u
     const int32_t* idx0 = good_idx ? good_idx + q0 * qt.idx_stride : nullptr;
     SwArgs a{queries + (size_t)q0 * query_stride, tpt * 32, idx0, g0, n_targets,
              ascii, delim, skip, out + q0 * out_stride, gap_a, gap_b, tickets + q0};
+    a.order = order;
     return launch_stream(a, mode, &qt, stream);
   };
   const int n_paired = pair ? (n_queries & ~1) : 0;
@@ -400,6 +425,18 @@ extern "C" int sseqs_sw_scan_queries(int affine, int n_queries, int tpt, const u
     if (st != SSEQS_OK) return st;
   }
   return SSEQS_OK;
+}
+
+extern "C" int sseqs_sw_scan_queries(int affine, int n_queries, int tpt, const uint8_t* queries,
+                                     int64_t query_stride, const int32_t* query_lens,
+                                     const int32_t* good_idx, int64_t idx_stride, int32_t g0,
+                                     int64_t n_targets,
+                                     const uint8_t* ascii, const int32_t* delim, int skip,
+                                     int32_t* out, int64_t out_stride, int gap_a, int gap_b,
+                                     uint32_t* tickets, cudaStream_t stream) {
+  return sseqs_sw_scan_queries_ordered(affine, n_queries, tpt, queries, query_stride, query_lens,
+                                       good_idx, idx_stride, g0, n_targets, nullptr, ascii, delim,
+                                       skip, out, out_stride, gap_a, gap_b, tickets, stream);
 }
 
 extern "C" int sseqs_sw_set_query_pairing(int tpt, int on) {

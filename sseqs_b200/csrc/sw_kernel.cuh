@@ -93,6 +93,8 @@ struct SwArgs {
   int32_t* out2;          // both: affine scores (out: linear)
   int skip2;              // both: the affine windows start this many (0 or 1)
                           // bytes after the linear ones
+  const int32_t* order;   // fast kernel: the targets in the order they are taken
+                          // (a permutation of 0 .. n-1; nullable: as they stand)
 };
 
 // Several queries of the same stripe width in one launch: blockIdx.y picks
@@ -571,27 +573,35 @@ __global__ void __launch_bounds__(Shape<TPT, W, MODE>::threads, Shape<TPT, W, MO
   // sizes CH so that every group gets several chunks.
   // The host splits launches so that n < 2^30: target indices and the
   // counter (which overshoots n by at most two grabs per group) fit 32 bits.
+  //
+  // With `order` (by length, the longest first) the launch ends on short targets
+  // instead of whatever stands last, and the groups of a warp, which wait for one
+  // another where a target ends, reach their ends together.  Measured on B200
+  // (lengths 30..1000, fused kernel): 100k targets at a 200-residue query 1.75 ->
+  // 1.38 ms, 500k 7.43 -> 6.59; affine at 858 residues 100k 3.45 -> 3.19, 500k
+  // 15.1 -> 14.7.
   const int CH = a.chunk;
   const int n = (int)a.n;
   unsigned pre_raw = 0;   // leader only: start of the prefetched chunk
   auto issue_grab = [&]() {
     if (gl == 0) pre_raw = atomicAdd(a.ticket, (unsigned)CH);
   };
-  int c_hi;               // end of the chunk the sequence is in
-  auto take_chunk = [&]() -> int {
-    const int c = (int)__shfl_sync(gmask, pre_raw, leader);
-    c_hi = c < n - CH ? c + CH : n;
-    if (c < n) issue_grab();
-    return c;
-  };
-  auto successor = [&](int x) -> int {   // next target after x (>= n: none)
-    return x + 1 < c_hi ? x + 1 : take_chunk();
+  int c_next = 0, c_hi = 0;              // what is left of the current chunk
+  auto successor = [&]() -> int {        // next target of the group (n: none)
+    if (c_next >= c_hi) {
+      c_next = (int)__shfl_sync(gmask, pre_raw, leader);
+      if (c_next >= n) return n;
+      c_hi = c_next < n - CH ? c_next + CH : n;
+      issue_grab();
+    }
+    const int at = c_next++;
+    return a.order ? __ldg(a.order + at) : at;
   };
 
   Win cur, nxt;
   int t, tn = 0;
   bool active = false, nxt_ok = false;
-  auto start_at = [&](int tt) {   // first target with rows at or after tt
+  auto start_at = [&](int tt) {   // first target with rows from tt on
     t = tt;
     while (t < n) {
       cur = window_of(a, t);
@@ -601,12 +611,12 @@ __global__ void __launch_bounds__(Shape<TPT, W, MODE>::threads, Shape<TPT, W, MO
         if constexpr (MODE == kBoth) a.out2[t] = cur.res;
         if constexpr (PAIR) if (writeB) outB[t] = cur.res;
       }
-      t = successor(t);
+      t = successor();
     }
     active = t < n;
     nxt_ok = false;
     if (active) {
-      tn = successor(t);
+      tn = successor();
       if (tn < n) { nxt = window_of(a, tn); nxt_ok = true; }
     }
   };
@@ -622,7 +632,7 @@ __global__ void __launch_bounds__(Shape<TPT, W, MODE>::threads, Shape<TPT, W, MO
     return best;
   };
   issue_grab();
-  start_at(take_chunk());
+  start_at(successor());
   if (active) classes(fetch(cur.pos, cur.end), cur.pos, cur.end, true);
 
   while (__any_sync(0xffffffffu, active)) {
@@ -662,7 +672,7 @@ __global__ void __launch_bounds__(Shape<TPT, W, MODE>::threads, Shape<TPT, W, MO
         if (pf_nxt) {
           t = tn;
           cur = nxt;
-          tn = successor(t);
+          tn = successor();
           nxt_ok = tn < n;
           if (nxt_ok) nxt = window_of(a, tn);
           classes(pf, cur.pos, cur.end, true);

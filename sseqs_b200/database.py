@@ -23,6 +23,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
+from . import select
 from ._lib import check, lib, ptr, stream_ptr, workspace
 
 CHUNK_BYTES = 1_000_000_000
@@ -41,6 +42,9 @@ class Batch:
     maxlen: int
     n_segments: int
     n_residues: int
+    # segments 1 .. n_segments-2, the targets of a whole-batch scan, from the
+    # longest to the shortest (select.length_order; target t is segment t + 1)
+    order: torch.Tensor | None = None
 
 
 class Database:
@@ -109,8 +113,9 @@ class Database:
         if m == 0:
             return
         self.n_residues += res
+        order = select.length_order(delim, m - 2, g0=1) if m > 2 else None
         self.batches.append(Batch(ci, j, ascii, n_sym, delim, seg_index[:m], lengths[:m],
-                                  offsets[:m], maxlen, m, res))
+                                  offsets[:m], maxlen, m, res, order))
 
     @classmethod
     def from_file(cls, path: str, chunks: int | None = None, bs: int = CHUNK_BYTES,

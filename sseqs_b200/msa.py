@@ -119,6 +119,13 @@ def search_batch(q_enc: torch.Tensor, query: str, batch, bi: int, *, top_fft=200
             stats.add("t_fft", t1 - t0)
             stats.add("t_topk1", stats.clock() - t1)
     t_sw0 = stats.clock() if stats is not None else 0.0
+
+    def order_of(idx):
+        # up to this many targets every lane group of a launch takes one
+        # or two, and two more launches to sort them would not pay
+        return (select.length_order(batch.delim, idx.numel(), good_idx=idx)
+                if idx.numel() > 8192 else None)
+
     Lq = q_enc.numel()
     k2 = n_c // top_sw
     if top_sw == 1 and tune.fused(Lq):
@@ -126,7 +133,8 @@ def search_batch(q_enc: torch.Tensor, query: str, batch, bi: int, *, top_fft=200
         # the two calls below)
         if timer is not None:
             timer("both", True)
-        tgt = dict(g0=1, n_targets=n_c) if cand is None else dict(good_idx=cand)
+        tgt = (dict(g0=1, n_targets=n_c, order=batch.order) if cand is None
+               else dict(good_idx=cand, order=order_of(cand)))
         lin, aff = _sw.sw_scan_both(q_enc, batch.ascii, batch.delim, affine_skip=1, gap=-1,
                                     gap_open=11, gap_extend=1, **tgt)
         if timer is not None:
@@ -135,10 +143,10 @@ def search_batch(q_enc: torch.Tensor, query: str, batch, bi: int, *, top_fft=200
     else:
         if cand is None:
             lin = _sw.sw_scan(q_enc, batch.ascii, batch.delim, affine=False, g0=1,
-                              n_targets=n_c, skip=0, gap_a=-1)
+                              n_targets=n_c, skip=0, gap_a=-1, order=batch.order)
         else:
             lin = _sw.sw_scan(q_enc, batch.ascii, batch.delim, affine=False, good_idx=cand,
-                              skip=0, gap_a=-1)
+                              skip=0, gap_a=-1, order=order_of(cand))
         if k2 <= 0:
             if stats is not None:
                 stats.add("t_sw", stats.clock() - t_sw0)
@@ -152,10 +160,11 @@ def search_batch(q_enc: torch.Tensor, query: str, batch, bi: int, *, top_fft=200
             timer("affine", True)
         if cand2 is None:
             aff = _sw.sw_scan(q_enc, batch.ascii, batch.delim, affine=True, g0=1, n_targets=k2,
-                              skip=1, gap_a=11, gap_b=1)
+                              skip=1, gap_a=11, gap_b=1, order=batch.order)
         else:
+            cand2 = cand2.to(torch.int32)
             aff = _sw.sw_scan(q_enc, batch.ascii, batch.delim, affine=True, good_idx=cand2,
-                              skip=1, gap_a=11, gap_b=1)
+                              skip=1, gap_a=11, gap_b=1, order=order_of(cand2))
         if timer is not None:
             timer("affine", False)
     # torch.topk raises when top_sw_affine exceeds the list (msa.py:335);

@@ -89,3 +89,16 @@ def topk_indices(values: torch.Tensor, k: int, out: torch.Tensor | None = None,
     check(L.sseqs_topk(ptr(values), kt, n, k, ptr(out), ptr(ws), ws.numel(), stream_ptr()),
           "topk")
     return out[:k]
+
+
+def length_order(delim: torch.Tensor, n: int, *, good_idx: torch.Tensor | None = None,
+                 g0: int = 0) -> torch.Tensor:
+    """The order (int32, a permutation of 0 .. n-1) that takes targets
+    ``good_idx`` (or ``g0 .. g0+n-1``) from the longest window to the shortest, in
+    steps of 8 residues; for the ``order`` of the score scans."""
+    L = lib()
+    out = torch.empty(max(int(n), 1), dtype=torch.int32, device=delim.device)
+    ws = workspace(L.sseqs_length_order_workspace_bytes(), delim.device)
+    check(L.sseqs_length_order(ptr(delim), ptr(good_idx), int(g0), int(n), ptr(out), ptr(ws),
+                               ws.numel(), stream_ptr()), "length_order")
+    return out[:n]

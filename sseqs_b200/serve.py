@@ -135,7 +135,7 @@ class GpuExecutor:
                 batched.sw_scan_queries(self.q, self.lens[:len(grp)], tpt, batch.ascii,
                                         batch.delim, affine=True, g0=1, n_targets=n, skip=1,
                                         gap_a=self.gaps[0], gap_b=self.gaps[1], out=sc,
-                                        tickets=self.tickets)
+                                        tickets=self.tickets, order=batch.order)
                 for j, i in enumerate(grp):
                     row = sc[j, :n]
                     p = select.topk_indices(row, k, out=self.idx, ws=self.ws)

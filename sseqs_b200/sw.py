@@ -63,17 +63,28 @@ def sw_cuda_affine(query_indices_tensor: torch.Tensor, good_idx: torch.Tensor,
     return out
 
 
+def _order(order: torch.Tensor | None, n: int) -> int | None:
+    """Address of an order of ``n`` targets."""
+    if order is None:
+        return None
+    if order.dtype != torch.int32 or order.numel() != n or not order.is_contiguous():
+        raise ValueError("order: one contiguous int32 per target")
+    return ptr(order)
+
+
 def sw_scan(query_idx: torch.Tensor, ascii: torch.Tensor, delim: torch.Tensor, *,
             affine: bool, good_idx: torch.Tensor | None = None, g0: int = 0,
             n_targets: int | None = None, skip: int = 0, gap_a: int = -1, gap_b: int = 0,
-            out: torch.Tensor | None = None) -> torch.Tensor:
+            out: torch.Tensor | None = None,
+            order: torch.Tensor | None = None) -> torch.Tensor:
     """Scores of database segments of one batch held in HBM.
 
     Segment g is the bytes between the '@' at ``delim[g-1]`` and ``delim[g]``;
     targets are ``good_idx`` (or ``g0 .. g0+n_targets-1``); the first ``skip``
     bytes of every segment are not scored.  ``skip=0`` with the linear gap is
     the call at sseqs/msa.py:313-319, ``skip=1`` with open/extend the one at
-    sseqs/msa.py:327-332.
+    sseqs/msa.py:327-332.  ``order`` (``select.length_order`` of the targets)
+    is the order the targets are taken in; scores do not depend on it.
     """
     if good_idx is not None:
         good_idx = _i32(good_idx)
@@ -82,16 +93,17 @@ def sw_scan(query_idx: torch.Tensor, ascii: torch.Tensor, delim: torch.Tensor, *
         n = int(n_targets)
     if out is None:
         out = torch.empty(n, dtype=torch.int32, device=ascii.device)
-    check(lib().sseqs_sw_scan(1 if affine else 0, ptr(query_idx), query_idx.numel(),
-                              ptr(good_idx), int(g0), n, ptr(ascii), ptr(delim), int(skip),
-                              ptr(out), int(gap_a), int(gap_b), stream_ptr()), "sw_scan")
+    check(lib().sseqs_sw_scan_ordered(1 if affine else 0, ptr(query_idx), query_idx.numel(),
+                                      ptr(good_idx), int(g0), n, _order(order, n), ptr(ascii),
+                                      ptr(delim), int(skip), ptr(out), int(gap_a), int(gap_b),
+                                      stream_ptr()), "sw_scan")
     return out
 
 
 def sw_scan_both(query_idx: torch.Tensor, ascii: torch.Tensor, delim: torch.Tensor, *,
                  good_idx: torch.Tensor | None = None, g0: int = 0,
                  n_targets: int | None = None, affine_skip: int = 1, gap: int = -1,
-                 gap_open: int = 11, gap_extend: int = 1):
+                 gap_open: int = 11, gap_extend: int = 1, order: torch.Tensor | None = None):
     """Linear (windows of ``sw_scan`` with skip 0) and affine (windows
     ``affine_skip`` bytes later) scores of the same targets in one pass:
     returns ``(linear, affine)``, each equal to its own ``sw_scan`` call."""
@@ -102,9 +114,10 @@ def sw_scan_both(query_idx: torch.Tensor, ascii: torch.Tensor, delim: torch.Tens
         n = int(n_targets)
     lin = torch.empty(n, dtype=torch.int32, device=ascii.device)
     aff = torch.empty(n, dtype=torch.int32, device=ascii.device)
-    check(lib().sseqs_sw_scan_both(ptr(query_idx), query_idx.numel(), ptr(good_idx), int(g0), n,
-                                   ptr(ascii), ptr(delim), int(affine_skip), ptr(lin), ptr(aff),
-                                   int(gap), int(gap_open), int(gap_extend), stream_ptr()),
+    check(lib().sseqs_sw_scan_both_ordered(ptr(query_idx), query_idx.numel(), ptr(good_idx),
+                                           int(g0), n, _order(order, n), ptr(ascii), ptr(delim),
+                                           int(affine_skip), ptr(lin), ptr(aff), int(gap),
+                                           int(gap_open), int(gap_extend), stream_ptr()),
           "sw_scan_both")
     return lin, aff
 
