@@ -446,6 +446,11 @@ int sseqs_pair_loss(const float* emb, int D, const int32_t* ia, const int32_t* i
 int sseqs_pool_backward(const float* emb, const float* dE, const float* inv_norm,
                         const int64_t* start, const int32_t* len, int n_seqs, int D,
                         const void* Z, void* dZ, void* G, cudaStream_t stream);
+/* Rows p with row_mask[p] == 0 of the bf16 [P x D] arrays a and b (nullable) to
+ * zero; 16-byte aligned, D a multiple of 8. */
+int sseqs_zero_rows(const uint8_t* row_mask, int64_t P, int D, void* a, void* b,
+                    cudaStream_t stream);
+
 /* db[c] += sum over the P rows of dZ[p][c]. */
 int sseqs_bias_grad(const void* dZ, int64_t P, int D, float* db, cudaStream_t stream);
 /* Adam step of a conv weight W[Cout][5][Cin] (fp32 w, m, v) from dWT

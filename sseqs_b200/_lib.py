@@ -80,6 +80,7 @@ _SIGNATURES = {
     "sseqs_pool_normalize": (_I, [_P, _I, _P, _P, _I, _P, _P, _P, _P]),
     "sseqs_pair_loss": (_I, [_P, _I, _P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "sseqs_pool_backward": (_I, [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _P]),
+    "sseqs_zero_rows": (_I, [_P, _I64, _I, _P, _P, _P]),
     "sseqs_bias_grad": (_I, [_P, _I64, _I, _P, _P]),
     "sseqs_adam_conv": (_I, [_P, _P, _P, _P, _I, _I, _F, _F, _F, _F, _I, _P, _P, _P]),
     "sseqs_adam_flat": (_I, [_P, _P, _P, _P, _I64, _F, _F, _F, _F, _I, _P, _P]),
@@ -159,6 +160,22 @@ def to_device(t: torch.Tensor, device="cuda") -> torch.Tensor:
 def to_host(t: torch.Tensor):
     transfer_bytes["d2h"] += t.numel() * t.element_size()
     return t.cpu().numpy()
+
+
+def to_host_many(tensors: list) -> list:
+    """``to_host`` of several device tensors: copies into page-locked memory
+    (torch's caching host allocator), queued together and waited for once."""
+    if not all(t.is_cuda for t in tensors):
+        return [to_host(t) for t in tensors]
+    out = []
+    for t in tensors:
+        transfer_bytes["d2h"] += t.numel() * t.element_size()
+        h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
+        h.copy_(t, non_blocking=True)
+        out.append(h)
+    if tensors:
+        torch.cuda.current_stream(tensors[0].device).synchronize()
+    return [h.numpy() for h in out]
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:

@@ -208,8 +208,9 @@ class Embedder:
         ``forward(..., train=True)``); returns them as a dict."""
         lay, emb, inv = self._cache
         bufs, P, L = self._bufs, lay.P, lib()
-        bufs.dZ[3][2:2 + P].zero_()
-        bufs.G[3][2:2 + P].zero_()
+        # pool_backward writes the sequences' rows; those between them are zero
+        check(L.sseqs_zero_rows(ptr(lay.mask), P, D, _base(bufs.dZ[3]), _base(bufs.G[3]),
+                                stream_ptr()), "zero_rows")
         check(L.sseqs_pool_backward(ptr(emb), ptr(dE), ptr(inv), ptr(lay.start),
                                     ptr(lay.length), lay.n, D, _base(bufs.Z[3]),
                                     _base(bufs.dZ[3]), _base(bufs.G[3]), stream_ptr()),

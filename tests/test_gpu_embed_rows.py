@@ -89,3 +89,18 @@ def test_pool_backward_forms_agree(with_g):
             _lib.ptr(z), _lib.ptr(dZ), _lib.ptr(G) if with_g else None, _lib.stream_ptr()))
         outs.append((dZ, G))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("P,D,both", [(1, 256, True), (31, 256, False), (33, 8, True),
+                                      (5000, 256, True)])
+def test_zero_rows(P, D, both):
+    from sseqs_b200 import _lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(P)
+    mask = (torch.rand(P, generator=g, device="cuda") > 0.4).to(torch.uint8)
+    a, b = (torch.ones(P + 1, D, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _lib.check(_lib.lib().sseqs_zero_rows(_lib.ptr(mask), P, D, _lib.ptr(a),
+                                          _lib.ptr(b) if both else None, _lib.stream_ptr()))
+    want = torch.cat([mask, mask.new_ones(1)])[:, None].expand(P + 1, D).to(torch.bfloat16)
+    assert torch.equal(a, want)
+    assert torch.equal(b, want if both else torch.ones_like(b))
