@@ -11,7 +11,7 @@ import ctypes
 
 import numpy as np
 
-from ._lib import check, lib, to_host
+from ._lib import check, lib, to_host_many
 from .sw import backtrack
 
 
@@ -59,9 +59,10 @@ def a3m_text_raw(query: str, results: list) -> str:
     in the same order (the same ``np.argsort`` of the same scores, the same
     first-occurrence placement).  Its case rule is str.upper/str.lower for
     ASCII; inputs holding other bytes take the string path of ``a3m_text``."""
-    host = [(to_host(r.best), to_host(r.info), to_host(r.q_al), to_host(r.t_al), r.cap)
-            for r in results]
-    if not query.isascii() or any((q >= 128).any() or (t >= 128).any() for _, _, q, t, _ in host):
+    flat = to_host_many([x for r in results for x in (r.best, r.info, r.q_al, r.t_al)])
+    host = [(*flat[4 * i:4 * i + 4], r.cap) for i, r in enumerate(results)]
+    if not query.isascii() or any(q.max(initial=0) >= 128 or t.max(initial=0) >= 128
+                                  for _, _, q, t, _ in host):
         return a3m_text(query, [d for r in results for d in r.to_dicts()])
     head = f">original_query\n{query}\n"
     if not host:
