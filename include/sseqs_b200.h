@@ -335,8 +335,9 @@ int64_t sseqs_launch_count(void);
 
 /* ----------------------------------------------------------- tuning */
 /* The score kernel has two lane layouts for stripe widths tpt =
- * ceil(query_len/32) <= 16: narrow (wide = 0, default) and wide (wide = 1:
- * twice the columns per lane, twice the targets per warp).  Selects the one
+ * ceil(query_len/32) <= 16 (linear: <= 29): narrow (wide = 0) and wide (wide =
+ * 1: twice the columns per lane, twice the targets per warp).  Where none is
+ * set, the width and the number of targets decide.  Selects the one
  * used for (affine, tpt) -- affine 0 linear, 1 affine, 2 the fused pass, 3
  * the query-pair kernel of sseqs_sw_scan_queries; both give identical
  * scores.  No reference

@@ -95,12 +95,32 @@ const Tables& tables() {
 struct Cache {
   std::mutex mu;
   int max_blocks[2][2][kModes][64][64] = {};  // [gaps][variant][mode][TPT-1][device]
-  int variant[kModes][64] = {};            // chosen variant per [mode][TPT-1]
+  int variant[kModes][64];                 // variant set by the caller per [mode][TPT-1], or -1
   bool pairing[64] = {};                   // per [TPT-1]: batched affine launches pair queries
 };
 Cache& cache() {
   static Cache c;
+  static std::once_flag once;
+  std::call_once(once, [] { std::fill(&c.variant[0][0], &c.variant[0][0] + kModes * 64, -1); });
   return c;
+}
+
+// The lane layout of a launch of n targets where none was set (the autotuner
+// sets one): `groups` lane groups of the narrow layout hold targets at once.
+// Measured on B200 at every width (targets of 30..1000 residues; narrow time over
+// wide).  150k targets, the longest first: linear 1.03-1.23 at widths 5-29 (8:
+// 0.99), affine 1.01-1.08 at 5-16, fused 1.01-1.10 at 6-16 (12: 0.97), below
+// 1 at narrower ones.  30k targets and fewer: 0.5-1.0, as the wide layout's rows take longer
+// and half the lanes have no target -- except the linear kernel from width 19
+// on while every target has a group to itself: 1.4-1.6 at 1400 targets (the wide
+// layout fetches 8 rows at a time there, the narrow one 4), 0.8 at 6000.
+int default_variant(int mode, int tpt, int64_t n, int64_t groups) {
+  if (n >= 8 * groups) {
+    if (mode == kLin) return tpt >= 5 && tpt <= 29 && tpt != 8;
+    if (mode == kAff) return tpt >= 5 && tpt <= 16;
+    if (mode == kBoth) return tpt >= 6 && tpt <= 16 && tpt != 12;
+  }
+  return mode == kLin && tpt >= 19 && tpt <= 29 && 2 * n <= groups;
 }
 
 // Target counters of the streaming kernel: every launch takes the next slot
@@ -138,24 +158,36 @@ int launch_stream(SwArgs a, int mode, const QueryTable* qt, cudaStream_t stream)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return SSEQS_ERR_CUDA;
   const int gaps = default_gaps(mode, a) ? 1 : 0;
-  int blocks_per_sm, var;
+  int blocks_per_sm;
   const KernelInfo* kp;
   {
     std::lock_guard<std::mutex> lk(cache().mu);
-    var = cache().variant[mode][tpt - 1];
-    kp = &tables().k[gaps][var][mode][tpt - 1];
-    int& mb = cache().max_blocks[gaps][var][mode][tpt - 1][dev];
-    if (mb == 0) {
-      if (cudaFuncSetAttribute((const void*)kp->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kp->smem) != cudaSuccess)
-        return SSEQS_ERR_CUDA;
-      int nb = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void*)kp->fn, kp->threads,
-                                                        kp->smem) != cudaSuccess || nb < 1)
-        return SSEQS_ERR_CUDA;
-      mb = nb;
+    // resident blocks per SM of a variant's kernel (0: an error)
+    auto blocks_of = [&](int var) -> int {
+      const KernelInfo& k = tables().k[gaps][var][mode][tpt - 1];
+      int& mb = cache().max_blocks[gaps][var][mode][tpt - 1][dev];
+      if (mb == 0) {
+        int nb = 0;
+        if (cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)k.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void*)k.fn, k.threads,
+                                                          k.smem) != cudaSuccess || nb < 1)
+          return 0;
+        mb = nb;
+      }
+      return mb;
+    };
+    int var = cache().variant[mode][tpt - 1];
+    if (var < 0) {
+      const int nb = blocks_of(0);
+      if (nb == 0) return SSEQS_ERR_CUDA;
+      const int64_t groups = (int64_t)device_sm_count() * nb *
+                             tables().k[gaps][0][mode][tpt - 1].groups_per_block;
+      var = default_variant(mode, tpt, a.n * (qt ? qt->n : 1), groups);
     }
-    blocks_per_sm = mb;
+    kp = &tables().k[gaps][var][mode][tpt - 1];
+    blocks_per_sm = blocks_of(var);
+    if (blocks_per_sm == 0) return SSEQS_ERR_CUDA;
   }
   const KernelInfo& k = *kp;
   const int64_t full = (int64_t)device_sm_count() * blocks_per_sm;
@@ -474,7 +506,7 @@ extern "C" int sseqs_sw_set_variant(int affine, int tpt, int wide) {
 extern "C" int sseqs_sw_get_variant(int affine, int tpt) {
   if (tpt < 1 || tpt > 64 || affine < 0 || affine >= kModes) return -1;
   std::lock_guard<std::mutex> lk(cache().mu);
-  return cache().variant[affine][tpt - 1];
+  return std::max(0, cache().variant[affine][tpt - 1]);
 }
 
 extern "C" int sseqs_sw_variant_words(int affine, int tpt, int wide) {

@@ -106,6 +106,10 @@ class Database:
         ws2 = workspace(L.sseqs_segments_workspace_bytes(nd + 1), dev)
         check(L.sseqs_segments(eff, ptr(delim), nd, trailing, ptr(seg_index), ptr(lengths),
                                ptr(offsets), ptr(info[2:]), ptr(ws2), ws2.numel(), st), "segments")
+        # the scan order, for the usual batch without empty segments (queued before
+        # the read below, after which everything is complete)
+        nseg = nd + trailing
+        order = select.length_order(delim, nseg - 2, g0=1) if nseg > 2 else None
         # a batch that is nearly full keeps its decoded buffer, a mostly empty
         # one a copy of the part that is used
         ascii = full[:eff] if 16 * (n_sym - eff) <= n_sym else full[:eff].clone()
@@ -113,7 +117,9 @@ class Database:
         if m == 0:
             return
         self.n_residues += res
-        order = select.length_order(delim, m - 2, g0=1) if m > 2 else None
+        if m != nseg:
+            order = select.length_order(delim, m - 2, g0=1) if m > 2 else None
+            torch.cuda.current_stream(dev).synchronize()
         self.batches.append(Batch(ci, j, ascii, n_sym, delim, seg_index[:m], lengths[:m],
                                   offsets[:m], maxlen, m, res, order))
 

@@ -800,12 +800,16 @@ class LearnedIndex:
                 plan.append((tpt, len(grp), m, pos_off, q_off))
                 pos_off += len(grp) * m
                 q_off += len(grp)
+        pos = torch.from_numpy(np.concatenate(pos_parts)).to(dev)
         # each query's candidates from the longest to the shortest, the order in which
         # the score kernel ends on short ones (8 queries of 32768 candidates: the
-        # seven score launches 8.2 -> 6.9 ms, the sort 0.06)
-        key = qid.to(torch.int32) * 65536 + (65535 - ulen.clamp(max=65535)[inv]).to(torch.int32)
-        by_len = torch.argsort(key) if nq < 32768 else torch.arange(n, device=dev)
-        pos = by_len[torch.from_numpy(np.concatenate(pos_parts)).to(dev)]
+        # seven score launches 8.2 -> 6.9 ms).  The sort takes about 0.1 ms, so it
+        # is left out where lists are short (a lane group then takes one or two
+        # of a query's targets) or few
+        if 65536 <= n and int(per_q.max()) > 8192 and nq < 32768:
+            key = (qid.to(torch.int32) * 65536 +
+                   (65535 - ulen.clamp(max=65535)[inv]).to(torch.int32))
+            pos = torch.argsort(key)[pos]
         lq = torch.from_numpy(np.concatenate(qid_parts)).to(dev)
         idx_all = inv[pos].to(torch.int32)
         qbuf = torch.zeros((nq, batched.MAX_QUERY), dtype=torch.uint8, device=dev)

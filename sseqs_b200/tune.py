@@ -59,12 +59,15 @@ def fused(query_len: int) -> bool:
 
 def _time(q, batch, mode, n, reps):
     sw = importlib.import_module("sseqs_b200.sw")
+    # a whole batch is scanned in its order, as the searches do
+    order = batch.order if n == batch.n_segments - 2 else None
     if mode == 2:
         def run():
-            sw.sw_scan_both(q, batch.ascii, batch.delim, g0=1, n_targets=n, affine_skip=1)
+            sw.sw_scan_both(q, batch.ascii, batch.delim, g0=1, n_targets=n, affine_skip=1,
+                            order=order)
     else:
         kw = dict(affine=mode == 1, g0=1, n_targets=n, skip=mode, gap_a=11 if mode else -1,
-                  gap_b=1)
+                  gap_b=1, order=order)
         out = torch.empty(n, dtype=torch.int32, device=batch.ascii.device)
 
         def run():
@@ -148,7 +151,8 @@ def autotune_pairing(query_lengths, batch, max_segments: int = 200_000, reps: in
         def run():
             batched.sw_scan_queries(q, lens, tpt, batch.ascii, batch.delim, affine=True, g0=1,
                                     n_targets=n, skip=1, gap_a=11, gap_b=1, out=out,
-                                    tickets=tickets)
+                                    tickets=tickets,
+                                    order=batch.order if n == batch.n_segments - 2 else None)
 
         def time_it():
             run()
