@@ -2180,33 +2180,6 @@ __global__ void layout_kernel(const uint8_t* ascii, const int64_t* off, const in
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = ascii_class(src[i]);
 }
 
-// Per row of x [rows][n]: the k-th largest value (k >= 1, k <= n <= 8192),
-// by a bitonic sort of the row in shared memory.
-constexpr int kKthMax = 8192;
-__global__ void __launch_bounds__(1024) kth_largest_kernel(const float* x, int n, int k,
-                                                           float* out) {
-  __shared__ float v[kKthMax];
-  const float* row = x + (int64_t)blockIdx.x * n;
-  int size = 1;
-  while (size < n) size <<= 1;
-  for (int i = threadIdx.x; i < size; i += blockDim.x) v[i] = i < n ? row[i] : -INFINITY;
-  __syncthreads();
-  for (int len = 2; len <= size; len <<= 1) {
-    for (int stride = len >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < size; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool desc = (i & len) == 0;     // descending runs first
-          const float a = v[i], b = v[j];
-          if (desc ? (a < b) : (a > b)) { v[i] = b; v[j] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = v[k - 1];
-}
-
 int grid_for(int64_t work, int threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads,
                                                     (int64_t)device_sm_count() * 16));
@@ -2750,14 +2723,5 @@ extern "C" int sseqs_embed_layout(const uint8_t* ascii, const int64_t* off, cons
     return SSEQS_ERR_ARG;
   if (n_seqs == 0) return SSEQS_OK;
   { layout_kernel<<<n_seqs, 128, 0, stream>>>(ascii, off, len, row0, cls); count_launches(1); }
-  return status_of(cudaGetLastError());
-}
-
-extern "C" int sseqs_kth_largest_rows(const float* x, int rows, int n, int k, float* out,
-                                      cudaStream_t stream) {
-  if (rows < 0 || n < 1 || n > kKthMax || k < 1 || k > n) return SSEQS_ERR_ARG;
-  if (rows == 0) return SSEQS_OK;
-  if (!x || !out) return SSEQS_ERR_ARG;
-  { kth_largest_kernel<<<rows, 1024, 0, stream>>>(x, n, k, out); count_launches(1); }
   return status_of(cudaGetLastError());
 }
