@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kSmallThreads)
 
 // Per row of x [rows][n]: the k-th largest value (1 <= k <= n <= kSmallN / 2), by
 // the passes of the one-block top-k on the row in registers.  8 rows of 8192:
-// 90 us as a bitonic sort in shared memory, now KTHFIG.
+// 90 us as a bitonic sort in shared memory, now 9.
 constexpr int kKthItems = 8, kKthMax = kSmallThreads * kKthItems;
 __global__ void __launch_bounds__(kSmallThreads)
     kth_largest_kernel(const float* x, int n, int k, float* out) {

@@ -95,6 +95,7 @@ struct SwArgs {
                           // bytes after the linear ones
   const int32_t* order;   // fast kernel: the targets in the order they are taken
                           // (a permutation of 0 .. n-1; nullable: as they stand)
+  int active_warps;       // fast kernel: warps of a block that take targets
 };
 
 // Several queries of the same stripe width in one launch: blockIdx.y picks
@@ -357,6 +358,9 @@ __global__ void __launch_bounds__(Shape<TPT, W, MODE>::threads, Shape<TPT, W, MO
     prof[i] = word;
   }
   __syncthreads();
+  // few targets: the launch spreads them over all SMs instead of filling blocks
+  // (a warp's rows take longer the more warps share its scheduler)
+  if ((int)(threadIdx.x >> 5) >= a.active_warps) return;
   const uint32_t* profL = prof;
   const uint32_t* profA = prof + (MODE == kBoth ? kNumCls * L::CLS : 0);
 

@@ -806,9 +806,8 @@ class LearnedIndex:
         # seven score launches 8.2 -> 6.9 ms).  The sort takes about 0.1 ms, so it
         # is left out where lists are short (a lane group then takes one or two
         # of a query's targets) or few
-        if 65536 <= n and int(per_q.max()) > 8192 and nq < 32768:
-            key = (qid.to(torch.int32) * 65536 +
-                   (65535 - ulen.clamp(max=65535)[inv]).to(torch.int32))
+        if n >= 65536 and int(per_q.max()) > 8192:
+            key = qid * 65536 + (65535 - ulen.clamp(max=65535)[inv])
             pos = torch.argsort(key)[pos]
         lq = torch.from_numpy(np.concatenate(qid_parts)).to(dev)
         idx_all = inv[pos].to(torch.int32)

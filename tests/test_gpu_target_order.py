@@ -81,3 +81,20 @@ def test_scans_do_not_depend_on_the_order(Lq):
             tune.set_query_pairing(tpt, pair)
     with pytest.raises(ValueError):
         sw.sw_scan(q, a, d, order=orders[0][:-1], **kw)
+
+
+@pytest.mark.parametrize("Lq", [20, 60, 150, 300, 500, 860])
+def test_few_targets_spread_over_blocks(Lq):
+    """Launches around a warp's, a block's and an SM round's number of targets
+    score as one launch over all of them does."""
+    sw = importlib.import_module("sseqs_b200.sw")
+    n = 9000
+    a, d, _ = _batch(n + 2, Lq + 1, hi=60)
+    q = _query(Lq, Lq)
+    kw = dict(affine=True, skip=1, gap_a=11, gap_b=1, g0=1)
+    aff = sw.sw_scan(q, a, d, n_targets=n, **kw)
+    lin = sw.sw_scan(q, a, d, affine=False, gap_a=-1, g0=1, n_targets=n)
+    for m in (1, 2, 3, 31, 33, 63, 65, 127, 129, 591, 593, 1183, 1185, 2367, 2369, 4737):
+        assert torch.equal(sw.sw_scan(q, a, d, n_targets=m, **kw), aff[:m])
+        both = sw.sw_scan_both(q, a, d, g0=1, n_targets=m)
+        assert torch.equal(both[0], lin[:m]) and torch.equal(both[1], aff[:m])
