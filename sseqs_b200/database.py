@@ -27,6 +27,7 @@ from . import select
 from ._lib import check, lib, ptr, stream_ptr, workspace
 
 CHUNK_BYTES = 1_000_000_000
+DECODE_ON = "cuda"         # where chunks are decoded: the current CUDA device
 
 
 @dataclass
@@ -72,10 +73,13 @@ class Database:
                 raise ValueError("chunk size must be a multiple of bs (sseqs/msa.py:216)")
             if self.packed is not None:
                 self.packed.append(ch)
+            # the kernels take addresses: contiguous bytes on the device whose
+            # stream they run on (a strided, expanded or host-held chunk is copied)
+            src = ch.to(device=DECODE_ON).contiguous()
             for j in range(ch.numel() // self.bs):
-                self._add_batch(ci, j, ch)
+                self._add_batch(ci, j, src)
             self.n_chunks += 1
-            del ch
+            del ch, src
 
     def _add_batch(self, ci, j, ch):
         n_sym = int(self.bs * 8 / 5)

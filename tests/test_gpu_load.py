@@ -55,3 +55,32 @@ def test_batches_match_restatement(kind, bs):
         assert (b.maxlen, b.n_segments, b.n_residues) == (
             seg["lengths"].max(), seg["lengths"].size, seg["lengths"].sum())
     assert db.n_residues == sum(int((a != 64).sum()) for _, a in want)
+
+
+@pytest.mark.parametrize("form", ["strided", "column", "rows", "host"])
+def test_views_of_a_chunk_load_as_its_contiguous_copy(form):
+    from sseqs_b200.database import Database
+    rng = np.random.default_rng(3)
+    bs = 5120
+    chunk = torch.from_numpy(np.concatenate(
+        [O.xbit_compress(_symbols("ends", bs * 8 // 5, rng)) for _ in range(2)])).cuda()
+    wide = torch.full((chunk.numel(), 3), 0xff, dtype=torch.uint8, device="cuda")
+    wide[:, 1] = chunk
+    view = {"strided": wide.reshape(-1)[1::3], "column": wide[:, 1], "rows": chunk.view(2, -1),
+            "host": chunk}[form]
+    want = Database([chunk], bs=bs).batches
+    got = Database([view], bs=bs, device="cpu" if form == "host" else "cuda").batches
+    assert len(got) == len(want) == 2
+    for g, w in zip(got, want):
+        assert (g.maxlen, g.n_segments, g.n_residues) == (w.maxlen, w.n_segments, w.n_residues)
+        for f in ("ascii", "delim", "seg_index", "lengths", "offsets"):
+            assert torch.equal(getattr(g, f), getattr(w, f)), f
+
+
+def test_an_expanded_chunk_loads_as_its_contiguous_copy():
+    from sseqs_b200.database import Database
+    one = torch.full((1,), 0b00100001, dtype=torch.uint8, device="cuda")
+    bs = 5120
+    got, want = (Database([c], bs=bs).batches[0] for c in
+                 (one.expand(bs), one.expand(bs).contiguous()))
+    assert torch.equal(got.ascii, want.ascii) and torch.equal(got.delim, want.delim)
