@@ -164,7 +164,8 @@ def to_host(t: torch.Tensor):
 
 def to_host_many(tensors: list) -> list:
     """``to_host`` of several device tensors: copies into page-locked memory
-    (torch's caching host allocator), queued together and waited for once."""
+    (torch's caching host allocator), queued together and waited for once on
+    each device that holds one."""
     if not all(t.is_cuda for t in tensors):
         return [to_host(t) for t in tensors]
     out = []
@@ -173,8 +174,8 @@ def to_host_many(tensors: list) -> list:
         h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
         h.copy_(t, non_blocking=True)
         out.append(h)
-    if tensors:
-        torch.cuda.current_stream(tensors[0].device).synchronize()
+    for dev in dict.fromkeys(t.device for t in tensors):
+        torch.cuda.current_stream(dev).synchronize()
     return [h.numpy() for h in out]
 
 
