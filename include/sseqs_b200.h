@@ -311,12 +311,22 @@ int sseqs_a3m_rows(const char* query, int64_t query_len, int64_t n_rows, const i
  * + lengths[s]); lut_a / lut_b are float [k][21] (k <= 20).  Replaces
  * launch_warp_corr (sseqs/filter.cu:161-395 with kernels
  * sseqs/filter.cu:92-159 and sseqs/fft.cu:17-415, wrapper
- * sseqs/filter_bind.cpp:20-64); computed in fp32. */
+ * sseqs/filter_bind.cpp:20-64).  Ranks k <= 4 multiply fp16-rounded look-up
+ * entries on the tensor cores and sum in fp32; higher ranks form each query
+ * profile entry in fp32, round it to fp16 and sum in fp32.
+ * A tensor-core launch whose bounded waits run out (the unit did not answer in
+ * time) still returns SSEQS_OK: segments that it could not score hold the fp16
+ * NaN 0x7fff, and the count that sseqs_prefilter_failures reads grows. */
 size_t sseqs_prefilter_workspace_bytes(int n, int k);
 int sseqs_prefilter(const uint8_t* ascii, const int64_t* offsets, const int32_t* lengths,
                     int64_t n_segments, const uint8_t* query_pos_reversed, int query_len,
                     const float* lut_a, const float* lut_b, int k, int n, void* out,
                     void* workspace, size_t ws_bytes, cudaStream_t stream);
+/* Copies to *out (device or page-locked host memory), in the order of `stream`,
+ * the number of prefilter waits that have run out on the current device since
+ * the library was loaded.  It is never cleared: a caller compares it with the
+ * value before its launches.  No reference counterpart. */
+int sseqs_prefilter_failures(uint32_t* out, cudaStream_t stream);
 
 /* --------------------------------------------------------- diagnostics */
 /* Measured int16x2 DPX issue rate of this GPU: runs a fixed kernel of

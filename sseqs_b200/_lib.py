@@ -64,6 +64,7 @@ _SIGNATURES = {
     "sseqs_a3m_rows": (_I, [_P, _I64, _I64, _P, _P, _P, _P, _P, _P, _I64, _P]),
     "sseqs_prefilter_workspace_bytes": (_SZ, [_I, _I]),
     "sseqs_prefilter": (_I, [_P, _P, _P, _I64, _P, _I, _P, _P, _I, _I, _P, _P, _SZ, _P]),
+    "sseqs_prefilter_failures": (_I, [_P, _P]),
     "sseqs_dpx_peak": (_I, [_P, ctypes.POINTER(_D), _P]),
     "sseqs_launch_count": (_I64, []),
     "sseqs_int16x2_peak": (_I, [_P, ctypes.POINTER(_D), _P]),

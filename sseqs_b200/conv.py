@@ -2,7 +2,8 @@
 
 ``prefilter_luts`` is the query-weighted SVD of BLOSUM62 of
 sseqs/msa.py:110-145 (same numpy calls, so the same tables); the scores come
-from ``csrc/prefilter.cu`` (fp32 FFTs, fp16 output).  ``warp_corr`` keeps the
+from ``csrc/prefilter.cu`` (the correlation summed directly, fp16 factors, fp32
+sums, fp16 output).  ``warp_corr`` keeps the
 call shape of sseqs/filter_bind.cpp:20-81 and fills ``corr`` in place.
 
 Supported transform lengths are 64..2048.  The reference computes no scores
@@ -10,6 +11,8 @@ Supported transform lengths are 64..2048.  The reference computes no scores
 is computed at 64 and N = 2048 is computed.
 """
 from __future__ import annotations
+
+import threading
 
 import numpy as np
 import torch
@@ -89,6 +92,44 @@ def prefilter_batch(query: str, batch, luts: Luts, fft_rank: int = 4) -> torch.T
     n = transform_length(len(query), batch.maxlen)
     return prefilter_scores(luts, batch.ascii, batch.offsets, batch.lengths, batch.n_segments,
                             n, fft_rank)
+
+
+_failures_seen: dict = {}
+_failures_lock = threading.Lock()
+
+
+def _copy_failures() -> torch.Tensor:
+    """The current device's count of failed prefilter waits, copied behind the
+    work queued on the current stream (complete when the stream has been waited for)."""
+    out = torch.empty(1, dtype=torch.int32, pin_memory=True)
+    check(lib().sseqs_prefilter_failures(ptr(out), stream_ptr()), "prefilter_failures")
+    return out
+
+
+class FailureWatch:
+    """Tells whether a prefilter launch made since this object was (on the current
+    device, by any thread) gave up a bounded wait, so that its scores are NaN.
+
+    ``queue`` behind the launches, ``check`` after results of the same stream have
+    been read: it costs no wait of its own then.  The count only grows, so
+    several searches at once all see a failure."""
+
+    def __init__(self):
+        self.device = torch.cuda.current_device()
+        self.before = _failures_seen.get(self.device, 0)
+        self.copy = None
+
+    def queue(self) -> None:
+        self.copy = _copy_failures()
+
+    def check(self) -> None:
+        torch.cuda.current_stream().synchronize()
+        now = int(self.copy.item())
+        with _failures_lock:
+            _failures_seen[self.device] = now
+        if now != self.before:
+            raise RuntimeError("prefilter: a bounded wait of the tensor-core kernel ran out; its "
+                               "scores are not valid")
 
 
 def warp_corr(corr, query_reversed_indices, weight_LUTS_A, W, flat, offsets, lengths, k,

@@ -2386,8 +2386,8 @@ extern "C" int sseqs_gemm_set_tensor_path(int tcgen05) {
   return SSEQS_OK;
 }
 
-// Reads and clears the flag a tcgen05 kernel (GEMM, selection, prefilter)
-// sets when one of its bounded waits runs out (synchronises the device).
+// Reads and clears the flag a tcgen05 kernel (GEMM, selection) sets when one of
+// its bounded waits runs out (synchronises the device).
 extern "C" int sseqs_gemm_error(int* out) {
   int* p = tc_error_flag();
   if (!p || !out) return SSEQS_ERR_ARG;

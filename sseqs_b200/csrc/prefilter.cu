@@ -43,6 +43,7 @@
 
 #include <algorithm>
 #include <array>
+#include <mutex>
 #include <utility>
 
 #include "tcgen05.cuh"
@@ -228,8 +229,8 @@ __global__ void __launch_bounds__(32 * PfShape<C>::WARPS) prefilter_kernel(PfArg
 // half of the tensor memory, so that the next one's products overlap its
 // epilogue; one of more than 512 (N = 2048) takes two passes.
 //
-// Waits are bounded; one that runs out sets the error flag, the CTA stops
-// and its segments score NaN.
+// Waits are bounded; one that runs out adds to the device's count of failures
+// (sseqs_prefilter_failures), the CTA stops and its segments score NaN.
 //
 // Measured (300k segments of 30..1000 residues, rank 4) against the per-warp
 // mma.sync form it replaced, which built every segment's Toeplitz operand
@@ -277,7 +278,7 @@ struct TcGroup {
   }
 };
 
-__global__ void __launch_bounds__(kTcThreads, 1) prefilter_tc_kernel(PfArgs a, int* err) {
+__global__ void __launch_bounds__(kTcThreads, 1) prefilter_tc_kernel(PfArgs a, unsigned* failures) {
   using namespace tc;
   extern __shared__ __align__(128) unsigned char pf_sm[];
   const int N = a.N, Lq = a.Lq, K = a.k;
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefilter_tc_kernel(PfArgs a, i
   const uint32_t tmem = tmem_base_s;
   auto fail = [&]() {
     abort_s = 1;
-    atomicExch(err, 1);
+    atomicAdd(failures, 1u);
   };
 
   // segment j of this CTA: runs of 32, gridDim.x apart
@@ -754,16 +755,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefilter_tc_kernel(PfArgs a, i
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTcCols));
 }
 
+// Waits of this kernel that ran out on each device since the library was loaded.
+// A count of its own, never cleared: searches in several threads compare it with
+// what it was before them, so that none takes another's failure away.
+__device__ unsigned g_pf_failures;
+
+unsigned* pf_failures() {
+  static std::mutex mu;
+  static unsigned* addr[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!addr[dev]) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_pf_failures) != cudaSuccess) return nullptr;
+    addr[dev] = static_cast<unsigned*>(p);
+  }
+  return addr[dev];
+}
+
 int launch_pf_tc(const PfArgs& a, cudaStream_t stream) {
-  int* err = tc_error_flag();
-  if (!err) return SSEQS_ERR_CUDA;
+  unsigned* failures = pf_failures();
+  if (!failures) return SSEQS_ERR_CUDA;
   const size_t smem = tc_smem(a.N);
   if (cudaFuncSetAttribute((const void*)prefilter_tc_kernel,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return SSEQS_ERR_CUDA;
   const int64_t groups = (a.n + kTcGroup - 1) / kTcGroup;
   const int grid = (int)std::min<int64_t>(groups, device_sm_count());
-  { prefilter_tc_kernel<<<grid, kTcThreads, smem, stream>>>(a, err); count_launches(1); }
+  { prefilter_tc_kernel<<<grid, kTcThreads, smem, stream>>>(a, failures); count_launches(1); }
   return status_of(cudaGetLastError());
 }
 
@@ -827,4 +847,11 @@ extern "C" int sseqs_prefilter(const uint8_t* ascii, const int64_t* offsets, con
   PfArgs a{ascii, offsets, lengths, n_segments, lut_a, lut_b, query_pos_reversed, query_len, k, n,
            reinterpret_cast<__half*>(out_scores)};
   return launch_pf(a, stream);
+}
+
+extern "C" int sseqs_prefilter_failures(uint32_t* out, cudaStream_t stream) {
+  if (!out) return SSEQS_ERR_ARG;
+  const unsigned* failures = pf_failures();
+  if (!failures) return SSEQS_ERR_CUDA;
+  return status_of(cudaMemcpyAsync(out, failures, sizeof(uint32_t), cudaMemcpyDefault, stream));
 }

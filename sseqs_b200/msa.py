@@ -287,6 +287,7 @@ def search(queries, db: Database | None = None, *, num_msas=4096, top_fft=200, t
     for query in queries:
         q_enc = _sw.encode_query(query, device=db.device)
         luts = conv.prefilter_luts(query, fft_rank) if top_fft != 1 else None
+        watch = conv.FailureWatch() if top_fft != 1 else None
         per = []
         for bi, batch in enumerate(db.batches):
             if abs(len(query) - batch.maxlen) > dlength:   # msa.py:252
@@ -294,7 +295,11 @@ def search(queries, db: Database | None = None, *, num_msas=4096, top_fft=200, t
             per.append(search_batch(q_enc, query, batch, bi, top_fft=top_fft, top_sw=top_sw,
                                     top_sw_affine=top_sw_affine, fft_rank=fft_rank, luts=luts,
                                     stats=stats, timer=timer))
+        if watch is not None:
+            watch.queue()
         out.append(rank_hits(query, per, num_msas))
+        if watch is not None:
+            watch.check()
         if per_batch_out is not None:
             per_batch_out.append(per)
     return out
