@@ -346,11 +346,11 @@ int64_t sseqs_launch_count(void);
 /* ----------------------------------------------------------- tuning */
 /* The score kernel has two lane layouts for stripe widths tpt =
  * ceil(query_len/32) <= 16 (linear: <= 29): narrow (wide = 0) and wide (wide =
- * 1: twice the columns per lane, twice the targets per warp).  Where none is
- * set, the width and the number of targets decide.  Selects the one
+ * 1: twice the columns per lane, twice the targets per warp).  Selects the one
  * used for (affine, tpt) -- affine 0 linear, 1 affine, 2 the fused pass, 3
- * the query-pair kernel of sseqs_sw_scan_queries; both give identical
- * scores.  No reference
+ * the query-pair kernel of sseqs_sw_scan_queries -- or, with wide = 2 (as a
+ * process starts), leaves it to the width and the number of targets of each
+ * launch.  Scores are the same either way.  No reference
  * counterpart (the autotuner of the batched path sets it). */
 int sseqs_sw_set_variant(int affine, int tpt, int wide);
 /* Whether sseqs_sw_scan_queries scores affine queries of stripe width tpt
@@ -361,8 +361,8 @@ int sseqs_sw_set_variant(int affine, int tpt, int wide);
  * scores one query at a time). */
 int sseqs_sw_set_query_pairing(int tpt, int on);
 int sseqs_sw_get_query_pairing(int tpt);
-/* The layout currently selected for (affine, tpt): 0 or 1; -1 if out of
- * range.  No reference counterpart. */
+/* What is set for (affine, tpt): 0, 1 or 2 as above, so that setting it again
+ * restores it; -1 if out of range.  No reference counterpart. */
 int sseqs_sw_get_variant(int affine, int tpt);
 /* int16x2 words per lane of a variant (for reports); -1 if out of range. */
 int sseqs_sw_variant_words(int affine, int tpt, int wide);

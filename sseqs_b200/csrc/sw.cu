@@ -92,16 +92,18 @@ const Tables& tables() {
   return t;
 }
 
+constexpr int kVariantAuto = 2;            // none set: default_variant decides
+
 struct Cache {
   std::mutex mu;
   int max_blocks[2][2][kModes][64][64] = {};  // [gaps][variant][mode][TPT-1][device]
-  int variant[kModes][64];                 // variant set by the caller per [mode][TPT-1], or -1
+  int variant[kModes][64];                 // variant set by the caller per [mode][TPT-1]
   bool pairing[64] = {};                   // per [TPT-1]: batched affine launches pair queries
 };
 Cache& cache() {
   static Cache c;
   static std::once_flag once;
-  std::call_once(once, [] { std::fill(&c.variant[0][0], &c.variant[0][0] + kModes * 64, -1); });
+  std::call_once(once, [] { std::fill(&c.variant[0][0], &c.variant[0][0] + kModes * 64, kVariantAuto); });
   return c;
 }
 
@@ -178,7 +180,7 @@ int launch_stream(SwArgs a, int mode, const QueryTable* qt, cudaStream_t stream)
       return mb;
     };
     int var = cache().variant[mode][tpt - 1];
-    if (var < 0) {
+    if (var == kVariantAuto) {
       const int nb = blocks_of(0);
       if (nb == 0) return SSEQS_ERR_CUDA;
       const int64_t groups = (int64_t)device_sm_count() * nb *
@@ -511,7 +513,7 @@ extern "C" int sseqs_int16x2_peak(uint32_t* sink, double* lane_ops_per_s, cudaSt
 }
 
 extern "C" int sseqs_sw_set_variant(int affine, int tpt, int wide) {
-  if (tpt < 1 || tpt > 64 || (wide != 0 && wide != 1) || affine < 0 || affine >= kModes)
+  if (tpt < 1 || tpt > 64 || wide < 0 || wide > kVariantAuto || affine < 0 || affine >= kModes)
     return SSEQS_ERR_ARG;
   std::lock_guard<std::mutex> lk(cache().mu);
   cache().variant[affine][tpt - 1] = wide;
@@ -521,7 +523,7 @@ extern "C" int sseqs_sw_set_variant(int affine, int tpt, int wide) {
 extern "C" int sseqs_sw_get_variant(int affine, int tpt) {
   if (tpt < 1 || tpt > 64 || affine < 0 || affine >= kModes) return -1;
   std::lock_guard<std::mutex> lk(cache().mu);
-  return std::max(0, cache().variant[affine][tpt - 1]);
+  return cache().variant[affine][tpt - 1];
 }
 
 extern "C" int sseqs_sw_variant_words(int affine, int tpt, int wide) {

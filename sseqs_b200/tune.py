@@ -33,13 +33,17 @@ MODES = ("linear", "affine", "both", "pair")
 MAX_FUSED_TPT = 23      # widths scored by the fused pass (wider: the two kernels)
 
 
+BY_SIZE = 2             # no layout set: width and number of targets decide
+
+
 def set_variant(affine, tpt: int, wide: int) -> None:
-    """``affine``: False/0 linear, True/1 affine, 2 the fused pass."""
+    """``affine``: False/0 linear, True/1 affine, 2 the fused pass, 3 the
+    query-pair kernel; ``wide``: 0 narrow, 1 wide, ``BY_SIZE`` neither set."""
     check(lib().sseqs_sw_set_variant(int(affine), int(tpt), int(wide)), "set_variant")
 
 
 def get_variant(affine, tpt: int) -> int:
-    """The layout selected for (kernel, tpt): 0 narrow, 1 wide."""
+    """What is set for (kernel, tpt): 0 narrow, 1 wide, ``BY_SIZE`` neither."""
     v = lib().sseqs_sw_get_variant(int(affine), int(tpt))
     if v < 0:
         raise ValueError(f"no score kernel for mode {affine}, width {tpt}")

@@ -98,3 +98,30 @@ def test_few_targets_spread_over_blocks(Lq):
         assert torch.equal(sw.sw_scan(q, a, d, n_targets=m, **kw), aff[:m])
         both = sw.sw_scan_both(q, a, d, g0=1, n_targets=m)
         assert torch.equal(both[0], lin[:m]) and torch.equal(both[1], aff[:m])
+
+
+@pytest.mark.parametrize("Lq", [20, 160, 250, 500, 700, 900])
+@pytest.mark.parametrize("n", [300, 9000, 200_000])
+def test_the_layout_by_size_scores_as_each_layout(Lq, n):
+    """With none set, few targets, many and a number between (past eight
+    lane groups' worth at 200000) score as both layouts do."""
+    sw = importlib.import_module("sseqs_b200.sw")
+    tune = importlib.import_module("sseqs_b200.tune")
+    a, d, _ = _batch(n + 2, Lq + n, hi=30 if n > 9000 else 300)
+    q = _query(Lq, Lq)
+    tpt = tune.tpt_of(Lq)
+    old = [tune.get_variant(m, tpt) for m in range(3)]
+    got = []
+    try:
+        for wide in (tune.BY_SIZE, 0, 1):
+            for m in range(3):
+                tune.set_variant(m, tpt, wide)
+            got.append((sw.sw_scan(q, a, d, affine=False, gap_a=-1, g0=1, n_targets=n),
+                        sw.sw_scan(q, a, d, affine=True, skip=1, gap_a=11, gap_b=1, g0=1,
+                                   n_targets=n), *sw.sw_scan_both(q, a, d, g0=1, n_targets=n)))
+    finally:
+        for m, v in enumerate(old):
+            tune.set_variant(m, tpt, v)
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert torch.equal(x, y)

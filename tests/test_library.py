@@ -112,6 +112,23 @@ def test_variant_selection_round_trips(built_lib):
     assert L.sseqs_sw_get_variant(4, 1) == -1 and L.sseqs_sw_get_variant(0, 65) == -1
 
 
+def test_an_unset_variant_can_be_put_back(built_lib):
+    """A process starts with no layout set; saving, setting and restoring one
+    leaves it unset, as does clearing it.  Host state only, no GPU."""
+    import subprocess
+    import sys
+    code = ("from sseqs_b200 import tune\n"
+            "before = [tune.get_variant(m, t) for m in range(4) for t in range(1, 65)]\n"
+            "assert set(before) == {tune.BY_SIZE}\n"
+            "for m in range(4):\n"
+            "    tune.set_variant(m, 5, 1)\n"
+            "    tune.set_variant(m, 5, before[0])\n"
+            "assert [tune.get_variant(m, t) for m in range(4) for t in range(1, 65)] == before\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
+    assert built_lib.sseqs_sw_set_variant(1, 9, 3) != 0
+    assert built_lib.sseqs_sw_set_variant(1, 9, -1) != 0
+
+
 def test_scan_both_argument_checks_without_a_gpu(built_lib):
     """sseqs_sw_scan_both rejects bad arguments on the host, before any
     CUDA call: a window shift other than 0/1, a missing output, a negative
