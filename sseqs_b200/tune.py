@@ -6,7 +6,8 @@ longer rows per lane group, or more targets per warp with twice the columns
 per lane.  Both give
 identical scores; which is faster depends on the width and on register
 pressure, so it is measured: each candidate scores a sample of database
-segments, timed with CUDA events on the current stream, and the faster one is
+segments, longest first as the searches take them, timed with CUDA events on
+the current stream, and the faster one is
 selected for that kernel (linear, affine, or the fused pass computing both)
 and width.  The batched affine launch can also score two queries per launch
 row (the query-pair kernel, ``sseqs_sw_set_query_pairing``); whether that is
@@ -61,10 +62,17 @@ def fused(query_len: int) -> bool:
     return 0 < tpt_of(query_len) <= MAX_FUSED_TPT
 
 
-def _time(q, batch, mode, n, reps):
+def _sample_order(batch, n: int):
+    """The order in which a search would take the first ``n`` targets of a batch
+    (the longest first; a batch that has no order is scanned as it stands)."""
+    if batch.order is None or n == batch.n_segments - 2:
+        return batch.order
+    from . import select
+    return select.length_order(batch.delim, n, g0=1)
+
+
+def _time(q, batch, mode, n, reps, order):
     sw = importlib.import_module("sseqs_b200.sw")
-    # a whole batch is scanned in its order, as the searches do
-    order = batch.order if n == batch.n_segments - 2 else None
     if mode == 2:
         def run():
             sw.sw_scan_both(q, batch.ascii, batch.delim, g0=1, n_targets=n, affine_skip=1,
@@ -99,6 +107,7 @@ def autotune(query_lengths, batch, max_segments: int = 200_000, reps: int = 2) -
         return dict(_chosen)
     gen = torch.Generator(device="cpu")
     gen.manual_seed(1)
+    order = _sample_order(batch, n)
     for tpt in sorted({tpt_of(L) for L in query_lengths if 0 < L}):
         q = None
         for mode, name in enumerate(MODES):
@@ -111,7 +120,7 @@ def autotune(query_lengths, batch, max_segments: int = 200_000, reps: int = 2) -
             t = []
             for wide in (0, 1):
                 set_variant(mode, tpt, wide)
-                t.append(_time(q, batch, mode, n, reps))
+                t.append(_time(q, batch, mode, n, reps, order))
             best = 0 if t[0] <= t[1] else 1
             set_variant(mode, tpt, best)
             _chosen[(name, tpt)] = best
@@ -144,6 +153,7 @@ def autotune_pairing(query_lengths, batch, max_segments: int = 200_000, reps: in
     gen = torch.Generator(device="cpu")
     gen.manual_seed(2)
     dev = batch.ascii.device
+    order = _sample_order(batch, n)
     for tpt in sorted({tpt_of(L) for L in query_lengths if 0 < L}):
         if ("pairing", tpt) in _chosen:
             continue
@@ -155,8 +165,7 @@ def autotune_pairing(query_lengths, batch, max_segments: int = 200_000, reps: in
         def run():
             batched.sw_scan_queries(q, lens, tpt, batch.ascii, batch.delim, affine=True, g0=1,
                                     n_targets=n, skip=1, gap_a=11, gap_b=1, out=out,
-                                    tickets=tickets,
-                                    order=batch.order if n == batch.n_segments - 2 else None)
+                                    tickets=tickets, order=order)
 
         def time_it():
             run()
