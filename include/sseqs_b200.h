@@ -351,8 +351,12 @@ int64_t sseqs_launch_count(void);
  * the query-pair kernel of sseqs_sw_scan_queries -- or, with wide = 2 (as a
  * process starts), leaves it to the width and the number of targets of each
  * launch.  Scores are the same either way.  No reference
- * counterpart (the autotuner of the batched path sets it). */
+ * counterpart. */
 int sseqs_sw_set_variant(int affine, int tpt, int wide);
+/* The layout (as above) for launches of min_targets targets or more, over all
+ * their queries, where sseqs_sw_set_variant has set none: what the autotuner
+ * of the batched path found on such launches.  No reference counterpart. */
+int sseqs_sw_tune_variant(int affine, int tpt, int wide, int64_t min_targets);
 /* Whether sseqs_sw_scan_queries scores affine queries of stripe width tpt
  * (0: every width) that share their targets two per launch row (on = 1) or
  * one (0, the default until the autotuner of the batched path has timed

@@ -69,6 +69,7 @@ _SIGNATURES = {
     "sseqs_launch_count": (_I64, []),
     "sseqs_int16x2_peak": (_I, [_P, ctypes.POINTER(_D), _P]),
     "sseqs_sw_set_variant": (_I, [_I, _I, _I]),
+    "sseqs_sw_tune_variant": (_I, [_I, _I, _I, _I64]),
     "sseqs_gemm_bf16": (_I, [_I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _P, _I64, _P, _P,
                              _P, _P, _P, _P]),
     "sseqs_gemm_set_tensor_path": (_I, [_I]),

@@ -98,12 +98,17 @@ struct Cache {
   std::mutex mu;
   int max_blocks[2][2][kModes][64][64] = {};  // [gaps][variant][mode][TPT-1][device]
   int variant[kModes][64];                 // variant set by the caller per [mode][TPT-1]
+  int tuned[kModes][64];                   // the autotuner's, for launches of tuned_from
+  int64_t tuned_from[kModes][64] = {};     // targets or more
   bool pairing[64] = {};                   // per [TPT-1]: batched affine launches pair queries
 };
 Cache& cache() {
   static Cache c;
   static std::once_flag once;
-  std::call_once(once, [] { std::fill(&c.variant[0][0], &c.variant[0][0] + kModes * 64, kVariantAuto); });
+  std::call_once(once, [] {
+    std::fill(&c.variant[0][0], &c.variant[0][0] + kModes * 64, kVariantAuto);
+    std::fill(&c.tuned[0][0], &c.tuned[0][0] + kModes * 64, kVariantAuto);
+  });
   return c;
 }
 
@@ -179,13 +184,17 @@ int launch_stream(SwArgs a, int mode, const QueryTable* qt, cudaStream_t stream)
       }
       return mb;
     };
+    // set, else tuned on launches like this one, else by size
+    const int64_t targets = a.n * (qt ? qt->n : 1);
     int var = cache().variant[mode][tpt - 1];
+    if (var == kVariantAuto && targets >= cache().tuned_from[mode][tpt - 1])
+      var = cache().tuned[mode][tpt - 1];
     if (var == kVariantAuto) {
       const int nb = blocks_of(0);
       if (nb == 0) return SSEQS_ERR_CUDA;
       const int64_t groups = (int64_t)device_sm_count() * nb *
                              tables().k[gaps][0][mode][tpt - 1].groups_per_block;
-      var = default_variant(mode, tpt, a.n * (qt ? qt->n : 1), groups);
+      var = default_variant(mode, tpt, targets, groups);
     }
     kp = &tables().k[gaps][var][mode][tpt - 1];
     blocks_per_sm = blocks_of(var);
@@ -517,6 +526,16 @@ extern "C" int sseqs_sw_set_variant(int affine, int tpt, int wide) {
     return SSEQS_ERR_ARG;
   std::lock_guard<std::mutex> lk(cache().mu);
   cache().variant[affine][tpt - 1] = wide;
+  return SSEQS_OK;
+}
+
+extern "C" int sseqs_sw_tune_variant(int affine, int tpt, int wide, int64_t min_targets) {
+  if (tpt < 1 || tpt > 64 || wide < 0 || wide > kVariantAuto || affine < 0 || affine >= kModes ||
+      min_targets < 0)
+    return SSEQS_ERR_ARG;
+  std::lock_guard<std::mutex> lk(cache().mu);
+  cache().tuned[affine][tpt - 1] = wide;
+  cache().tuned_from[affine][tpt - 1] = min_targets;
   return SSEQS_OK;
 }
 

@@ -13,7 +13,8 @@ and width.  The batched affine launch can also score two queries per launch
 row (the query-pair kernel, ``sseqs_sw_set_query_pairing``); whether that is
 faster depends on the width as well (it shares the per-row work, but doubles
 the profile in shared memory), so ``autotune_pairing`` times it against one
-query per row.  Choices are kept for the process.
+query per row.  Choices are kept for the process, for launches of the size
+they were timed at.
 """
 from __future__ import annotations
 
@@ -41,6 +42,16 @@ def set_variant(affine, tpt: int, wide: int) -> None:
     """``affine``: False/0 linear, True/1 affine, 2 the fused pass, 3 the
     query-pair kernel; ``wide``: 0 narrow, 1 wide, ``BY_SIZE`` neither set."""
     check(lib().sseqs_sw_set_variant(int(affine), int(tpt), int(wide)), "set_variant")
+
+
+def _keep(mode: int, tpt: int, wide: int, targets: int) -> None:
+    """Use the layout that was the faster one over ``targets`` targets in launches
+    of at least half as many.  A layout found at 200k targets is within 5% of the
+    other one at 100k; at 50k the wide one takes up to 1.3 times as long
+    (measured at eleven widths), so smaller launches go by size."""
+    set_variant(mode, tpt, BY_SIZE)
+    check(lib().sseqs_sw_tune_variant(int(mode), int(tpt), int(wide), targets // 2),
+          "tune_variant")
 
 
 def get_variant(affine, tpt: int) -> int:
@@ -122,7 +133,7 @@ def autotune(query_lengths, batch, max_segments: int = 200_000, reps: int = 2) -
                 set_variant(mode, tpt, wide)
                 t.append(_time(q, batch, mode, n, reps, order))
             best = 0 if t[0] <= t[1] else 1
-            set_variant(mode, tpt, best)
+            _keep(mode, tpt, best, n)
             _chosen[(name, tpt)] = best
     return dict(_chosen)
 
@@ -179,7 +190,7 @@ def autotune_pairing(query_lengths, batch, max_segments: int = 200_000, reps: in
             return e0.elapsed_time(e1) / reps
 
         set_query_pairing(tpt, False)
-        best_t, best = time_it(), (False, get_variant(3, tpt))
+        best_t, best = time_it(), (False, BY_SIZE)
         for wide in ((0, 1) if has_wide(3, tpt) else (0,)):
             set_query_pairing(tpt, True)
             set_variant(3, tpt, wide)
@@ -187,7 +198,7 @@ def autotune_pairing(query_lengths, batch, max_segments: int = 200_000, reps: in
             if t < best_t:
                 best_t, best = t, (True, wide)
         set_query_pairing(tpt, best[0])
-        set_variant(3, tpt, best[1])
+        _keep(3, tpt, best[1], n_queries * n)
         _chosen[("pairing", tpt)] = int(best[0])
         if best[0]:
             _chosen[("pair", tpt)] = best[1]

@@ -125,3 +125,24 @@ def test_the_layout_by_size_scores_as_each_layout(Lq, n):
     for other in got[1:]:
         for x, y in zip(got[0], other):
             assert torch.equal(x, y)
+
+
+def test_a_tuned_layout_scores_the_same_on_both_sides_of_its_line():
+    from sseqs_b200 import _lib
+    sw = importlib.import_module("sseqs_b200.sw")
+    tune = importlib.import_module("sseqs_b200.tune")
+    a, d, _ = _batch(4002, 3)
+    q = _query(150, 3)
+    old = tune.get_variant(1, 5)
+    kw = dict(affine=True, skip=1, gap_a=11, gap_b=1, g0=1)
+    try:
+        tune.set_variant(1, 5, 0)
+        want = sw.sw_scan(q, a, d, n_targets=4000, **kw)
+        tune.set_variant(1, 5, tune.BY_SIZE)
+        for wide in (0, 1):
+            _lib.check(_lib.lib().sseqs_sw_tune_variant(1, 5, wide, 2000))
+            for n in (1999, 2000, 4000):
+                assert torch.equal(sw.sw_scan(q, a, d, n_targets=n, **kw), want[:n])
+    finally:
+        _lib.check(_lib.lib().sseqs_sw_tune_variant(1, 5, tune.BY_SIZE, 0))
+        tune.set_variant(1, 5, old)
