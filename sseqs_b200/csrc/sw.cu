@@ -112,18 +112,21 @@ Cache& cache() {
   return c;
 }
 
-// The lane layout of a launch of n targets where none was set (the autotuner
-// sets one): `groups` lane groups of the narrow layout hold targets at once.
-// Measured on B200 at every width (targets of 30..1000 residues; narrow time over
-// wide).  150k targets, the longest first: linear 1.03-1.23 at widths 5-29 (8:
-// 0.99), affine 1.01-1.08 at 5-16, fused 1.01-1.10 at 6-16 (12: 0.97), below
-// 1 at narrower ones.  30k targets and fewer: 0.5-1.0, as the wide layout's rows take longer
-// and half the lanes have no target -- except the linear kernel from width 19
-// on while every target has a group to itself: 1.4-1.6 at 1400 targets (the wide
-// layout fetches 8 rows at a time there, the narrow one 4), 0.8 at 6000.
+// The lane layout of a launch of n targets where none was set or tuned: `groups`
+// lane groups of the narrow layout hold targets at once.
+// Measured on B200 over targets of log-normal lengths (30..1000), of 30..1000 and of
+// 60..200 residues, the longest first; narrow time over wide, repeats within 0.02
+// from 150k targets on.  At 150k and 250k: linear 1.02-1.21 at widths 5-29, affine
+// 1.04-1.17 at 5-16, fused 0.99-1.08 at 6-16 but for 0.98-0.99 at 12 in every
+// set (fused 5: 1.03-1.11, yet 0.95-1.05 at 100k; linear 4: 0.71-0.88).  At 50k
+// 0.81-1.18, as the wide layout's rows take longer and lanes run out of
+// targets sooner; the ratios cross 1 between 50k and 120k, about eight targets a
+// group.  The linear kernel from width 19 on is faster wide again while every target has
+// a group to itself (the wide layout fetches 8 rows at a time there, the narrow
+// one 4): 0.96-1.35 at 1000 targets, 1.04-1.72 at 2400, but 0.74-0.87 at 6000.
 int default_variant(int mode, int tpt, int64_t n, int64_t groups) {
   if (n >= 8 * groups) {
-    if (mode == kLin) return tpt >= 5 && tpt <= 29 && tpt != 8;
+    if (mode == kLin) return tpt >= 5 && tpt <= 29;
     if (mode == kAff) return tpt >= 5 && tpt <= 16;
     if (mode == kBoth) return tpt >= 6 && tpt <= 16 && tpt != 12;
   }
