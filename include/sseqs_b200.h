@@ -297,7 +297,8 @@ int sseqs_backtrack_affine(const uint8_t* query, int query_len, const uint8_t* t
  * row loop of to_a3m (sseqs/to_a3m.py:16-72).  *out_len receives the bytes
  * written to out; SSEQS_ERR_UNSUPPORTED when a fragment does not occur in
  * the query (the reference raises ValueError), SSEQS_ERR_CAPACITY when
- * out_cap is too small. */
+ * out_cap is less than the text of the kept rows.  Bytes of out past *out_len
+ * are scratch. */
 int sseqs_a3m_rows(const char* query, int64_t query_len, int64_t n_rows, const int64_t* order,
                    const uint8_t* const* q_rows, const uint8_t* const* t_rows,
                    const int32_t* lens, const int64_t* scores, char* out, int64_t out_cap,

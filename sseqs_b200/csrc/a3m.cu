@@ -29,7 +29,8 @@ inline int64_t find_first(const char* hay, int64_t n, const char* needle, int64_
   return -1;
 }
 
-// 64-bit hash of n bytes, 8 at a time (multiply and xor-shift).
+// 64-bit hash of n bytes, 8 at a time (multiply and xor-shift; the multiplier is
+// that of MurmurHash3's 64-bit finaliser, public domain).
 inline uint64_t hash_bytes(const char* p, size_t n) {
   uint64_t h = 0x9e3779b97f4a7c15ull ^ (uint64_t)n;
   auto mix = [&](uint64_t w) {
@@ -57,15 +58,12 @@ class RowSet {
   }
   bool insert(int64_t at, size_t n) {           // false: an equal row is there
     const uint64_t h = hash_bytes(base_ + at, n);
-    for (size_t k = h & (slots_.size() - 1);; k = (k + 1) & (slots_.size() - 1)) {
-      Slot& s = slots_[k];
-      if (s.at < 0) {
-        s = Slot{h, at, n};
-        return true;
-      }
-      if (s.hash == h && s.n == n && std::memcmp(base_ + s.at, base_ + at, n) == 0) return false;
-    }
+    Slot& s = find(base_ + at, n, h);
+    if (s.at >= 0) return false;
+    s = Slot{h, at, n};
+    return true;
   }
+  bool contains(const char* row, size_t n) { return find(row, n, hash_bytes(row, n)).at >= 0; }
 
  private:
   struct Slot {
@@ -73,6 +71,12 @@ class RowSet {
     int64_t at;
     size_t n;
   };
+  Slot& find(const char* row, size_t n, uint64_t h) {   // an equal row's slot, or a free one
+    for (size_t k = h & (slots_.size() - 1);; k = (k + 1) & (slots_.size() - 1)) {
+      Slot& s = slots_[k];
+      if (s.at < 0 || (s.hash == h && s.n == n && std::memcmp(base_ + s.at, row, n) == 0)) return s;
+    }
+  }
   const char* base_;
   std::vector<Slot> slots_;
 };
@@ -107,7 +111,7 @@ extern "C" int sseqs_a3m_rows(const char* query, int64_t query_len, int64_t n_ro
   *out_len = 0;
   try {
     RowSet seen(out, n_rows);
-    std::vector<char> compact;
+    std::vector<char> compact, spill;
     std::vector<int32_t> gaps;
     int64_t pos = 0;
     for (int64_t i = 0; i < n_rows; ++i) {
@@ -132,11 +136,15 @@ extern "C" int sseqs_a3m_rows(const char* query, int64_t query_len, int64_t n_ro
       // first occurrence, as str.find
       const int64_t q0 = m > 0 ? find_first(query, query_len, compact.data(), m) : 0;
       if (q0 < 0) return SSEQS_ERR_UNSUPPORTED;
-      // ">target_<i> score=<s>.0": at most 64 bytes
       const int64_t row_len = query_len - m + n;
-      if (pos + 64 + row_len + 1 > out_cap) return SSEQS_ERR_CAPACITY;
-      char* p = put(put(put(put(put(out + pos, ">target_"), i), " score="), scores[k]), ".0\n");
-      char* row = p;
+      char head[64];                                   // ">target_<i> score=<s>.0"
+      const char* head_end = put(put(put(put(put(head, ">target_"), i), " score="), scores[k]), ".0\n");
+      const int64_t head_len = head_end - head;
+      // a row that does not fit is an error only if it is kept
+      const bool fits = pos + head_len + row_len + 1 <= out_cap;
+      if (!fits) spill.resize((size_t)row_len);
+      char* row = fits ? out + pos + head_len : spill.data();
+      char* p = row;
       std::memset(p, '-', (size_t)q0);
       p += q0;
       // upper case over the row, then lower case where the query has a gap
@@ -149,7 +157,13 @@ extern "C" int sseqs_a3m_rows(const char* query, int64_t query_len, int64_t n_ro
       p += n;
       std::memset(p, '-', (size_t)(query_len - q0 - m));
       p += query_len - q0 - m;
-      if (at_sign || !seen.insert(row - out, (size_t)row_len)) continue;   // written over
+      if (at_sign) continue;                           // written over
+      if (!fits) {
+        if (seen.contains(row, (size_t)row_len)) continue;
+        return SSEQS_ERR_CAPACITY;
+      }
+      if (!seen.insert(row - out, (size_t)row_len)) continue;
+      std::memcpy(out + pos, head, (size_t)head_len);
       *p++ = '\n';
       pos = p - out;
     }

@@ -102,3 +102,39 @@ def test_sequence_helpers_keep_the_reference_layout():
     assert W == 4 and T.dtype == torch.int16 and lens.dtype == torch.int32
     assert T.tolist() == [[0, 65, 67, 0], [0, 87, 89, 86], [0, 0, 0, 0]]
     assert lens.tolist() == [3, 4, 1]
+
+
+@pytest.mark.parametrize("last", ["kept", "repeat", "at sign"])
+def test_rows_fill_a_buffer_of_their_own_size(last):
+    """sseqs_a3m_rows needs room for the rows it keeps and no more: a buffer of
+    exactly their text is enough, whatever is dropped after them; one byte less
+    is not.  Nothing is written past it."""
+    import ctypes
+    from sseqs_b200 import _lib
+    query = b"MKTAYIAKQRQISFVK"
+    rows = [(b"TAYIAK", b"TAYWAK"), (b"MKTA-Y", b"MRTAGY")]
+    if last == "repeat":
+        rows.append(rows[0])
+    if last == "at sign":
+        rows.append((query, b"MKTAYIA@QRQISFVK"))
+    n = len(rows)
+    text = b">target_0 score=30.0\n--TAYWAK--------\n>target_1 score=20.0\nMRTAgY-----------\n"
+    q, t = [[np.frombuffer(r[k], np.uint8).copy() for r in rows] for k in (0, 1)]
+    ptrs = [np.array([x.ctypes.data for x in v], np.uint64) for v in (q, t)]
+    lens = np.array([len(r[0]) for r in rows], np.int32)
+    scores = np.array([30, 20, 10][:n], np.int64)
+    order = np.arange(n, dtype=np.int64)
+
+    def write(cap):
+        out = np.full(cap + 64, 7, np.uint8)
+        got = ctypes.c_int64(-1)
+        st = _lib.lib().sseqs_a3m_rows(
+            query, ctypes.c_int64(len(query)), ctypes.c_int64(n),
+            *[ctypes.c_void_p(a.ctypes.data) for a in (order, *ptrs, lens, scores, out)],
+            ctypes.c_int64(cap), ctypes.byref(got))
+        assert (out[cap:] == 7).all()
+        return st, out[:max(got.value, 0)].tobytes()
+
+    assert write(len(text)) == (0, text)
+    assert write(len(text) + 200) == (0, text)
+    assert write(len(text) - 1)[0] == 5            # SSEQS_ERR_CAPACITY
