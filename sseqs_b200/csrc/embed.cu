@@ -2266,11 +2266,18 @@ static bool make_map_u8(CUtensorMap* map, const void* base, int64_t rows, int bo
          CUDA_SUCCESS;
 }
 
+// Whether rows of `n` elements, lda apart, are whole 64-column slabs of a matrix
+// with lda columns: an overlapping view that ends with a slab row (the boxes of one
+// that ends inside would read past the operand).
+static bool slab_view(int64_t lda, int64_t n) {
+  return lda >= 64 && lda < n && lda % 64 == 0 && n % lda == 0;
+}
+
 // The TMA-fed kernel applies when the operands' K tiles are boxes: A with
-// lda >= K (a plain matrix) or lda % 64 == 0 (an overlapping row view), B
+// lda >= K (a plain matrix) or an overlapping view of slabs, B
 // with ldb >= K; 16-byte aligned bases and strides (checked by the caller).
 static bool ws_applies(const GemmArgs& g) {
-  return (g.lda >= g.K || g.lda % TC_BK == 0) && g.ldb >= g.K && g.lda <= INT32_MAX &&
+  return (g.lda >= g.K || slab_view(g.lda, g.K)) && g.ldb >= g.K && g.lda <= INT32_MAX &&
          g.M + g.K / std::max<int64_t>(1, g.lda) < INT32_MAX;
 }
 
@@ -2329,8 +2336,8 @@ static bool conv_applies(const GemmArgs& g) {
   if (!al(g.C, 32) || !al(g.C2, 32) || !al(g.aux, 32) || !al(g.res, 32) || g.ldc % 16 != 0 ||
       !al(g.bias, 16))
     return false;
-  return g.lda < g.K && g.lda % 64 == 0 && g.lda / 64 <= CV_SLABS && g.K % g.lda == 0 &&
-         g.K / g.lda <= CV_MAX_TAPS && g.M >= (int64_t)512 * device_sm_count();
+  return slab_view(g.lda, g.K) && g.lda / 64 <= CV_SLABS && g.K / g.lda <= CV_MAX_TAPS &&
+         g.M >= (int64_t)512 * device_sm_count();
 }
 
 template <int EPI>
@@ -2351,13 +2358,13 @@ int launch_conv(const GemmArgs& g, cudaStream_t stream) {
   return status_of(cudaGetLastError());
 }
 
-// The MN-major kernel applies when 64-column boxes of A stay inside its rows
-// (a plain matrix, or an overlapping view with lda % 64 == 0) and C takes
-// 16-byte reductions.
+// The MN-major kernel applies when 64-column boxes of A stay inside its rows (a
+// plain matrix or a view of slabs) and C takes 16-byte reductions.
 static bool wg_applies(const GemmArgs& g) {
-  return g.N == 256 && g.K >= 64 && (g.lda >= g.M || g.lda % 64 == 0) && g.ldb >= 256 &&
-         g.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
-         g.M <= 256 * 65535 && g.K + g.M / std::max<int64_t>(1, g.lda) < INT32_MAX - 256;
+  return g.N == 256 && g.K >= 64 && (g.lda >= g.M || slab_view(g.lda, g.M)) && g.ldb >= 256 &&
+         g.lda <= INT32_MAX && g.ldb <= INT32_MAX && g.ldc % 4 == 0 &&
+         (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 && g.M <= 256 * 65535 &&
+         g.K + g.M / std::max<int64_t>(1, g.lda) < INT32_MAX - 256;
 }
 
 static int launch_wg(const GemmArgs& g, cudaStream_t stream) {

@@ -50,3 +50,22 @@ def test_slab_gemm_matches_64_bit_rows(M, lda, taps):
     # tanh.approx is within 2^-10.9 of tanh; the sum is rounded to bf16
     assert ((fused[rows].float() - y).abs() <= 2.0 ** -8 * y.abs() + 2.0 ** -11 * zb.abs() +
             1e-6).all()
+
+
+@pytest.mark.parametrize("M", [1000, FIRST + 129])
+@pytest.mark.parametrize("lda,K", [(128, 192), (64, 64), (192, 256), (0, 128), (8, 320)])
+def test_other_row_views_match_64_bits(M, lda, K):
+    """Views whose last row ends inside its slab (the operand ends with the
+    buffer), one row for every output (lda = 0), rows 8 elements apart."""
+    from sseqs_b200 import learned
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + lda + K)
+    X = torch.randn((M - 1) * lda + K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(256, K, generator=g, device="cuda").to(torch.bfloat16)
+    C = torch.zeros(M, 256, dtype=torch.bfloat16, device="cuda")
+    learned._gemm(0, 0, learned._EPI_BF16, M, 256, K, X.data_ptr(), lda, B.data_ptr(), K,
+                  C.data_ptr(), 256)
+    A = torch.as_strided(X, (M, K), (lda, 1)).double()
+    exp, size = A @ B.double().T, A.abs() @ B.double().abs().T
+    tol = 2.0 ** -8 * exp.abs() + K / 16 * 2.0 ** -22 * size
+    assert ((C.double() - exp).abs() <= tol).all()

@@ -69,3 +69,22 @@ def test_first_layer_gradients_match_64_bits(P):
     assert ((dWT.double() - torch.cat(exp_w)).abs()
             <= (rel + 21 * 2.0 ** -23) * torch.cat(size_w)).all()
     assert ((dE.double() - exp_e).abs() <= (rel + 1280 * 2.0 ** -23) * size_e).all()
+
+
+@pytest.mark.parametrize("M,lda,K", [(72, 64, 64), (136, 128, 96), (320, 256, 1056), (64, 0, 96),
+                                     (256, 8, 128)])
+def test_other_row_views_match_64_bits(M, lda, K):
+    """Views whose last row ends inside its slab (the operand ends with the
+    buffer, which holds no byte more), one row for every position (lda = 0), and
+    rows 8 elements apart."""
+    from sseqs_b200 import learned
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + lda + K)
+    buf = torch.randn((K - 1) * lda + M, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(K, 256, generator=g, device="cuda").to(torch.bfloat16)
+    C = torch.zeros(M, 256, device="cuda")
+    learned._gemm(1, 1, learned._EPI_F32_ADD, M, 256, K, buf.data_ptr(), lda, B.data_ptr(), 256,
+                  C.data_ptr(), 256)
+    A = torch.as_strided(buf, (K, M), (lda, 1)).double()
+    exp, size = A.T @ B.double(), A.abs().T @ B.double().abs()
+    assert ((C.double() - exp).abs() <= (K / 16 + 150) * 2.0 ** -23 * size).all()
