@@ -96,6 +96,11 @@ def length_order(delim: torch.Tensor, n: int, *, good_idx: torch.Tensor | None =
     """The order (int32, a permutation of 0 .. n-1) that takes targets
     ``good_idx`` (or ``g0 .. g0+n-1``) from the longest window to the shortest, in
     steps of 8 residues; for the ``order`` of the score scans."""
+    if good_idx is not None:
+        if good_idx.device != delim.device or good_idx.numel() < n:
+            raise ValueError("length_order: good_idx holds n targets, beside the delimiters")
+        # what the kernel reads; held here until its launch is queued
+        good_idx = good_idx.to(torch.int32).contiguous()
     L = lib()
     out = torch.empty(max(int(n), 1), dtype=torch.int32, device=delim.device)
     ws = workspace(L.sseqs_length_order_workspace_bytes(), delim.device)

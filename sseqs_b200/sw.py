@@ -67,8 +67,9 @@ def _order(order: torch.Tensor | None, n: int) -> int | None:
     """Address of an order of ``n`` targets."""
     if order is None:
         return None
-    if order.dtype != torch.int32 or order.numel() != n or not order.is_contiguous():
-        raise ValueError("order: one contiguous int32 per target")
+    if (order.dtype != torch.int32 or order.numel() != n or not order.is_contiguous() or
+            not order.is_cuda):
+        raise ValueError("order: one contiguous int32 per target, on the GPU")
     return ptr(order)
 
 
