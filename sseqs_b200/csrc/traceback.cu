@@ -72,9 +72,10 @@ constexpr int kTbRing = 128;                     // columns of a ring (a power o
 constexpr int kTbClasses = 21;
 // Scores are held times 4, the low two bits of a candidate for H naming its
 // state, so that one maximum decides both (ties: stop, M, Ix, Iy, in this order)
-// and the code is the maximum's low bits.
+// and the code is the maximum's low bits.  That leaves 2^29 for a score: gap
+// costs below 0 (bonuses) can go past it, and then scores are held as they are and
+// the state is found by comparisons (TAGGED false, chosen at the launch).
 constexpr int kTagStop = 3, kTagM = 2, kTagX = 1, kTagY = 0;
-constexpr int kNegIx = 4 * kNegBorder + kTagX, kNegIy = 4 * kNegBorder + kTagY;
 
 // Shared memory per warp: scores [class][lane] (4 int8 each), and the ring its
 // first lane reads.
@@ -84,8 +85,12 @@ __device__ __forceinline__ int byte_of(uint32_t w, int r) {      // sign-extende
   return (int)(w << (24 - 8 * r)) >> 24;
 }
 
-template <bool MATRIX>
+template <bool MATRIX, bool TAGGED>
 __global__ void __launch_bounds__(32 * kTbMaxWarps, MATRIX ? 2 : 4) traceback_kernel(TbArgs a) {
+  constexpr int SHIFT = TAGGED ? 2 : 0;
+  constexpr int M_TAG = TAGGED ? kTagM : 0, X_TAG = TAGGED ? kTagX : 0, Y_TAG = TAGGED ? kTagY : 0;
+  constexpr int kNegIx = (1 << SHIFT) * kNegBorder + X_TAG;
+  constexpr int kNegIy = (1 << SHIFT) * kNegBorder + Y_TAG;
   extern __shared__ int2 tb_sm[];
   __shared__ uint8_t scls[256];
   __shared__ int8_t sb62[400];
@@ -111,7 +116,8 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps, MATRIX ? 2 : 4) traceback_ke
   __syncthreads();
 
   const uint8_t* t = a.tbytes + a.toff[b];
-  const int ge = 4 * a.ge, open_x = kTagX - 4 * a.go, open_y = kTagY - 4 * a.go;
+  const int ge = (1 << SHIFT) * a.ge;
+  const int open_x = X_TAG - (1 << SHIFT) * a.go, open_y = Y_TAG - (1 << SHIFT) * a.go;
   const int own_phases = (Lt + 31 + 31) >> 5;         // a row block's Lt + 31 steps
   const int words = 2 * own_phases;                   // its code words
   uint4* dir = a.dir + (int64_t)b * a.dir_stride;
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps, MATRIX ? 2 : 4) traceback_ke
 #pragma unroll
         for (int r = 0; r < kTbRows; ++r) {
           const int s = (qc[r] >= 0 && c < kNumAA) ? sb62[qc[r] * 20 + c] : -5;
-          v |= (uint32_t)(uint8_t)(int8_t)(4 * s + kTagM) << (8 * r);
+          v |= (uint32_t)(uint8_t)(int8_t)((1 << SHIFT) * s + M_TAG) << (8 * r);
         }
         prof[c * 32 + lane] = v;
       }
@@ -197,15 +203,18 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps, MATRIX ? 2 : 4) traceback_ke
               // floor (tag 3) and M (2), Ix (1), Iy (0): the largest tagged value is
               // the cell's H and, in its low bits, the state that gave it
               const int sm = byte_of(sc, r);
-              const int m = __viaddmax_s32(diag, sm, kTagStop);
+              const int m = __viaddmax_s32(diag, sm, TAGGED ? kTagStop : 0);
               const int x = __viaddmax_s32(hu, open_x, xu - ge);
               const int y = __viaddmax_s32(hl[r], open_y, yl[r] - ge);
               const int v = __vimax3_s32(m, x, y);
-              const int h = v & ~3;
-              code[r] = (uint32_t)v;
+              const int h = TAGGED ? v & ~3 : v;
+              code[r] = TAGGED   ? (uint32_t)v
+                        : v == 0 ? (uint32_t)kTagStop
+                        : v == m ? (uint32_t)kTagM
+                                 : (uint32_t)(v == x ? kTagX : kTagY);
               if (h > rbest[r]) { rbest[r] = h; rbj[r] = j; }
               if constexpr (MATRIX) {
-                if (i0 + r < Lq) mf[(int64_t)(i0 + r + 1) * a.tcols + j] = (sm + diag) >> 2;
+                if (i0 + r < Lq) mf[(int64_t)(i0 + r + 1) * a.tcols + j] = (sm + diag) >> SHIFT;
               }
               diag = hl[r];
               hl[r] = h;
@@ -280,7 +289,7 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps, MATRIX ? 2 : 4) traceback_ke
       bestv = ov; bi = oi; bj = oj;
     }
   }
-  bestv >>= 2;
+  bestv >>= SHIFT;
   a.best[b] = bestv;
   int32_t* inf = a.info + (int64_t)b * 5;
   inf[0] = 0; inf[1] = -1; inf[2] = -1; inf[3] = -1; inf[4] = -1;
@@ -352,13 +361,19 @@ extern "C" int sseqs_backtrack_affine(const uint8_t* query, int query_len, const
                                         ~(uintptr_t)15);
   const int64_t ds = dir_tiles(query_len, max_target_len);
   int2* top = reinterpret_cast<int2*>(dir + (int64_t)B * ds);
-  // scores are held times 4: a gap cost past 2^26 is past every score all the same
-  auto cost = [](int g) { return std::max(-(1 << 26), std::min(1 << 26, g)); };
+  // The tagged form, unless a step's largest gain (11, or a gap that is a bonus) over
+  // the longest path could come near 2^26.  Below that a gap cost of 2^26 or more
+  // makes a state negative and less than its other source whatever its
+  // size, so larger ones are cut to it.
+  const int64_t gain = std::max<int64_t>({11, -(int64_t)gap_open, -(int64_t)gap_extend});
+  const bool tagged = gain * ((int64_t)query_len + max_target_len + 2) < (1 << 26) + kNegBorder;
+  auto cost = [&](int g) { return tagged ? std::min(1 << 26, g) : g; };
   TbArgs a{query, query_len, tbytes, toff, tlen, B, cost(gap_open), cost(gap_extend), dir, ds,
            top, (int64_t)max_target_len + 1, best, info, q_aligned, t_aligned, cap, m_full, tcols,
            max_target_len};
   const int warps = std::max(1, std::min(kTbMaxWarps, (query_len + kTbBlock - 1) / kTbBlock));
-  auto fn = m_full ? traceback_kernel<true> : traceback_kernel<false>;
+  auto fn = m_full ? (tagged ? traceback_kernel<true, true> : traceback_kernel<true, false>)
+                   : (tagged ? traceback_kernel<false, true> : traceback_kernel<false, false>);
   { fn<<<B, 32 * warps, warps * kTbWarpBytes, stream>>>(a); count_launches(1); }
   return status_of(cudaGetLastError());
 }

@@ -42,3 +42,53 @@ def test_matrix_at_block_edges():
                 Y[i, j] = max(H[i, j - 1] - 11, Y[i, j - 1] - 1)
                 H[i, j] = max(0, m, X[i, j], Y[i, j])
                 assert M[b, i, j] == m
+
+
+def _gotoh(query, target, go, ge):
+    """Best score and alignment of one pair in 64 bits, row by row: the first best
+    cell in query-major order, states in the order M, Ix, Iy."""
+    n, m = len(query), len(target)
+    H = np.zeros((n + 1, m + 1), np.int64)
+    M, X, Y = (np.full((n + 1, m + 1), -16384, np.int64) for _ in range(3))
+    for i in range(1, n + 1):
+        for j in range(1, m + 1):
+            s = O.BLOSUM62[O.AA_MAP[query[i - 1]], O.AA_MAP[target[j - 1]]]
+            M[i, j] = s + H[i - 1, j - 1]
+            X[i, j] = max(H[i - 1, j] - go, X[i - 1, j] - ge)
+            Y[i, j] = max(H[i, j - 1] - go, Y[i, j - 1] - ge)
+            H[i, j] = max(0, M[i, j], X[i, j], Y[i, j])
+    best = int(H.max())
+    i, j = np.unravel_index(int(H.argmax()), H.shape)
+    qa, ta = [], []
+    while i > 0 and j > 0 and H[i, j] > 0:
+        if H[i, j] == M[i, j]:
+            qa.append(query[i - 1])
+            ta.append(target[j - 1])
+            i, j = i - 1, j - 1
+        elif H[i, j] == X[i, j]:
+            qa.append(query[i - 1])
+            ta.append("-")
+            i -= 1
+        else:
+            qa.append("-")
+            ta.append(target[j - 1])
+            j -= 1
+    return best, "".join(reversed(qa)), "".join(reversed(ta))
+
+
+@pytest.mark.parametrize("gaps", [
+    (-1, -1), (11, -40), (-300_000, 5), (-210_000, -1), (-240_000, -240_000),
+    (-3_000_000, -3_000_000), (7, -3_000_000), (-3_000_000, 2), (1 << 27, -200_000),
+    (1 << 30, -6_000_000), (1 << 27, 1 << 27), (1 << 30, 1 << 30), (-2_000_000, 1 << 30)])
+def test_gap_costs_of_any_size_and_sign(gaps):
+    """Gaps that are bonuses, up to sums near the 32-bit range, and costs past
+    every score: each pair as a 64-bit restatement aligns it."""
+    from sseqs_b200.sw import backtrack
+    rng = np.random.default_rng(5)
+    query = rand_seq(rng, 133)
+    targets = [rand_seq(rng, 150), query[20:110], rand_seq(rng, 1), rand_seq(rng, 33) + query[:60]]
+    res = backtrack(query, targets, *gaps)
+    best = res.best.cpu().tolist()
+    for t, b, got in zip(targets, best, res.to_dicts()):
+        exp = _gotoh(query, t, *gaps)
+        assert (b, got["q_aligned"], got["t_aligned"]) == exp
