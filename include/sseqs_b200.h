@@ -425,12 +425,6 @@ int sseqs_embed_layout(const uint8_t* ascii, const int64_t* off, const int32_t* 
 int sseqs_embed_conv1_table(const uint8_t* cls, int64_t P, const float* T, const float* bias,
                             const uint8_t* row_mask, int D, void* Y, void* Z,
                             cudaStream_t stream);
-/* X[p][c] = E[cls[p]][c] (bf16, E [21][D]); 0 for padding rows. */
-int sseqs_embed_lookup(const uint8_t* cls, int64_t P, const void* E, int D, void* X,
-                       cudaStream_t stream);
-/* dE[cls[p]][c] += dX[p][c] (fp32 dE, bf16 dX). */
-int sseqs_embed_grad(const uint8_t* cls, int64_t P, const void* dX, int D, float* dE,
-                     cudaStream_t stream);
 /* Gradients through the first convolution and the residue embedding: with
  * G[t][k][co] = sum of dZ[p][co] over rows p with cls[p - 2 + t] == k (rows
  * outside [0, P) and classes >= 21 contribute nothing),
@@ -439,7 +433,7 @@ int sseqs_embed_grad(const uint8_t* cls, int64_t P, const void* dX, int D, float
  * cls uint8 [P]; dZ bf16 [P x D], D = 256; E bf16 [21 x cin]; Wf bf16
  * [cin][5][D] (the layout sseqs_adam_conv writes); G: workspace of 5 * 21 * D
  * floats, left holding the sums.  Stands for the weight- and data-gradient GEMMs of
- * that layer and sseqs_embed_grad. */
+ * that layer and the sum of its input gradients by class. */
 int sseqs_embed_conv1_grad(const uint8_t* cls, int64_t P, const void* dZ, int D, const void* E,
                            int cin, const void* Wf, float* G, float* dWT, float* dE,
                            cudaStream_t stream);

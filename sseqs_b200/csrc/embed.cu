@@ -1417,30 +1417,6 @@ __global__ void __launch_bounds__(32 * kConvWarps, 2)
   }
 }
 
-// X0[p][c] = E[cls[p]][c] for real rows (cls < 21), 0 for padding (cls 255).
-__global__ void embed_lookup_kernel(const uint8_t* cls, int64_t P, const __nv_bfloat16* E, int D,
-                                    __nv_bfloat16* X) {
-  const int64_t total = P * D;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / D;
-    const int c = (int)(i - p * D), k = cls[p];
-    X[i] = k < 21 ? E[k * D + c] : __float2bfloat16_rn(0.f);
-  }
-}
-
-// dE[cls[p]][c] += dX[p][c]
-__global__ void embed_grad_kernel(const uint8_t* cls, int64_t P, const __nv_bfloat16* dX, int D,
-                                  float* dE) {
-  const int64_t total = P * D;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / D;
-    const int c = (int)(i - p * D), k = cls[p];
-    if (k < 21) atomicAdd(dE + k * D + c, __bfloat162float(dX[i]));
-  }
-}
-
 // Gradients through the first convolution and the residue embedding.  The
 // layer's input rows are class embeddings, so both only need the sums of dZ by
 // class and tap, G[t][k] = sum of dZ[p] over the rows p with cls[p - 2 + t] == k:
@@ -2515,26 +2491,6 @@ extern "C" int sseqs_embed_conv1_table(const uint8_t* cls, int64_t P, const floa
   { conv1_table_kernel<<<grid, 256, smem, stream>>>(
         cls, P, T, bias, row_mask, D, static_cast<__nv_bfloat16*>(Y),
         static_cast<__nv_bfloat16*>(Z));
-    count_launches(1); }
-  return status_of(cudaGetLastError());
-}
-
-extern "C" int sseqs_embed_lookup(const uint8_t* cls, int64_t P, const void* E, int D, void* X,
-                                  cudaStream_t stream) {
-  if (P < 0 || D <= 0 || (P > 0 && (!cls || !E || !X))) return SSEQS_ERR_ARG;
-  if (P == 0) return SSEQS_OK;
-  { embed_lookup_kernel<<<grid_for(P * D, 256), 256, 0, stream>>>(
-        cls, P, static_cast<const __nv_bfloat16*>(E), D, static_cast<__nv_bfloat16*>(X));
-    count_launches(1); }
-  return status_of(cudaGetLastError());
-}
-
-extern "C" int sseqs_embed_grad(const uint8_t* cls, int64_t P, const void* dX, int D, float* dE,
-                                cudaStream_t stream) {
-  if (P < 0 || D <= 0 || (P > 0 && (!cls || !dX || !dE))) return SSEQS_ERR_ARG;
-  if (P == 0) return SSEQS_OK;
-  { embed_grad_kernel<<<grid_for(P * D, 256), 256, 0, stream>>>(
-        cls, P, static_cast<const __nv_bfloat16*>(dX), D, dE);
     count_launches(1); }
   return status_of(cudaGetLastError());
 }
