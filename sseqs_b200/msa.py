@@ -299,7 +299,7 @@ def search(queries, db: Database | None = None, *, num_msas=4096, top_fft=200, t
             watch.queue()
         out.append(rank_hits(query, per, num_msas))
         if watch is not None:
-            watch.check()
+            watch.check(waited=bool(out[-1]))      # the hits came to the host after it
         if per_batch_out is not None:
             per_batch_out.append(per)
     return out

@@ -17,7 +17,7 @@ def count(monkeypatch):
 
     class Stream:
         def synchronize(self):
-            pass
+            box["waits"] = box.get("waits", 0) + 1
 
     monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream())
@@ -49,6 +49,16 @@ def test_a_failed_prefilter_raises_once(count, monkeypatch):
     assert _search(monkeypatch, lambda bi: None) == [[]]      # an older failure is not this one's
     with pytest.raises(RuntimeError, match="prefilter"):
         _search(monkeypatch, fails)
+
+
+def test_the_count_is_read_only_after_a_wait(count, monkeypatch):
+    """Hits that were read waited for the copy queued before them; a search
+    without hits waits itself."""
+    _search(monkeypatch, lambda bi: None)
+    assert count["waits"] == 1
+    monkeypatch.setattr(M, "rank_hits", lambda *a: [("hit",)])
+    _search(monkeypatch, lambda bi: None)
+    assert count["waits"] == 1
 
 
 def test_without_a_prefilter_nothing_is_asked(count, monkeypatch):
