@@ -394,7 +394,7 @@ int sseqs_sw_variant_words(int affine, int tpt, int wide);
  * (a_t, b_t) = (0, 0).  row_mask
  * (nullable, uint8 per row of C): rows with 0 are written as 0 (epilogues
  * 1-3).  A, B 16-byte aligned, lda, ldb multiples of 8; a_t needs M % 8 ==
- * 0, b_t N % 8 == 0.  Tensor cores (mma.sync bf16, fp32 accumulation). */
+ * 0, b_t N % 8 == 0.  Tensor cores (bf16 products, fp32 accumulation). */
 int sseqs_gemm_bf16(int a_t, int b_t, int epilogue, int64_t M, int64_t N, int64_t K,
                     const void* A, int64_t lda, const void* B, int64_t ldb, void* C,
                     int64_t ldc, void* C2, const float* bias, const void* aux,
@@ -403,8 +403,10 @@ int sseqs_gemm_bf16(int a_t, int b_t, int epilogue, int64_t M, int64_t N, int64_
 /* sseqs_gemm_bf16 runs on the 5th-generation tensor cores (tcgen05.mma,
  * fp32 accumulators in tensor memory) when a_t = b_t = 0, N = 256, K is a
  * multiple of 64, ldc a multiple of 8, C/C2/aux/res 16-byte aligned and the
- * epilogue is 1, 2, 3, 5 or 6; otherwise on mma.sync.  set_tensor_path(0)
- * forces mma.sync (1 restores the default).  gemm_error reads and clears the
+ * epilogue is 1, 2, 3, 5 or 6; and when a_t = b_t = 1, epilogue 4, N = 256, K >= 64,
+ * lda >= M (or A a view of whole rows: lda a multiple of 64 that divides M), ldb >=
+ * 256, ldc a multiple of 4 and C 16-byte aligned; otherwise on mma.sync.
+ * set_tensor_path(0) forces mma.sync (1 restores the default).  gemm_error reads and clears the
  * flag a tcgen05 launch sets when one of its bounded waits ran out
  * (synchronous).  A set flag means the tensor-core unit did not answer in
  * time: the launch's output is invalid, and since its last operations were
