@@ -107,8 +107,9 @@ def _copy_failures() -> torch.Tensor:
 
 
 class FailureWatch:
-    """Tells whether a prefilter launch made since this object was (on the current
-    device, by any thread) gave up a bounded wait, so that its scores are NaN.
+    """Tells whether a prefilter launch on the current device gave up a bounded wait,
+    so that its scores are NaN: any launch, by any thread, since the last ``check``
+    before this object was made.
 
     ``queue`` behind the launches, ``check`` after results of the same stream have
     been read: no wait of its own then, and 6 us of host time in all.  The count
